@@ -479,121 +479,208 @@ namespace {
 // fewer resident blocks leave fewer graphs running at once).
 constexpr int SEG_BLOCK = 512;
 
+// Rows longer than SEG_HEAVY arcs are walked by every warp of the block
+// together, up to SEG_HEAVY_MAX of them per round.
+constexpr int SEG_HEAVY = 256, SEG_HEAVY_MAX = 32;
+// Frontier vertices whose rows a warp has in flight together.
+constexpr int SEG_GROUP = 8;
+
 struct SegShared {
   int32_t todo, level, minv, fcnt, ncnt;
   uint32_t g;
+  // peel_graph_smem: one slot per phase (scan or round) mod 3, reset one
+  // phase before it is used, one phase after it was last read
+  uint32_t cnt[3], mn[3], hcnt[3];
+  uint16_t heavy[SEG_HEAVY_MAX];
 };
 
 // Graphs of at most SEG_SMEM_N vertices keep their remaining degrees (16-bit
-// halves of 32-bit words, decremented by one atomic on the word: a degree
-// never falls below zero, so no borrow reaches the other half) and their
-// core numbers (16-bit, -1 while unpeeled) in shared memory: the rounds'
-// decrements and tests stay on the SM.  Their frontiers hold local ids.
+// halves of 32-bit words, decremented by one atomic on the word; bit 15 marks
+// a vertex that is queued or removed, whose further decrements change
+// nothing) and the order in which vertices are queued (16-bit local ids) in
+// shared memory.  The frontier of a round is a slice of that order.
 constexpr int SEG_SMEM_N = 16384;
+constexpr uint32_t SEG_GONE = 0x8000u;
 
-__device__ __forceinline__ int sdeg_get(const uint32_t *w, int i) {
-  return (int)((w[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu);
-}
-__device__ __forceinline__ int sdeg_dec(uint32_t *w, int i) {  // returns the old degree
-  const uint32_t sh = (uint32_t)(i & 1) * 16u;
-  return (int)((atomicSub(&w[i >> 1], 1u << sh) >> sh) & 0xFFFFu);
-}
-
-// One graph (local vertices 0..n-1 = union vertices vb..vb+n-1) with its
-// state in shared memory; the rounds and their numbering are those of the
-// global-memory path below.
+// One graph (local vertices 0..n-1 = union vertices vb..vb+n-1) peeled by one
+// block; the rounds and their numbering are those of the global-memory path
+// below.  What bounds it is the chain of dependent loads (row offsets, arcs)
+// of each round, so a warp takes up to SEG_GROUP frontier vertices at a time
+// and has their rows' first windows in flight together, one block barrier
+// ends the light rows of a round and one the long ones (long rows are spread
+// over the warps), and the tests and decrements stay on the SM.
 __device__ void peel_graph_smem(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
-                                int32_t *core, uint32_t *prio, int32_t *F0, int32_t *G0,
-                                int64_t vb, int n, uint32_t mg, uint32_t *sdeg, int16_t *score,
-                                SegShared &sh, PeelCtl *ctl) {
+                                int32_t *core, uint32_t *prio, int64_t vb, int n, uint32_t mg,
+                                uint32_t *sdeg, uint16_t *order, SegShared &sh, PeelCtl *ctl) {
   const int lane = (int)lane_id(), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = threadIdx.x; 2 * k < n; k += blockDim.x) {
+  const uint32_t lt = (1u << lane) - 1u;
+  const int words = (n + 1) >> 1;
+  for (int k = threadIdx.x; k < words; k += blockDim.x) {
     const int64_t v = vb + 2 * k;
-    const uint32_t d0 = (uint32_t)(rp[v + 1] - rp[v]);
-    const uint32_t d1 = 2 * k + 1 < n ? (uint32_t)(rp[v + 2] - rp[v + 1]) : 0u;
+    const int32_t r0 = rp[v], r1 = rp[v + 1], r2 = 2 * k + 1 < n ? rp[v + 2] : r1;
+    const uint32_t d0 = (uint32_t)min(r1 - r0, 0x7FFF);
+    const uint32_t d1 = 2 * k + 1 < n ? (uint32_t)min(r2 - r1, 0x7FFF) : 0xFFFFu;
     sdeg[k] = d0 | (d1 << 16);
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    score[i] = -1;
-    prio[vb + i] = mg;
-  }
-  if (threadIdx.x == 0) {
-    sh.todo = n;
-    sh.level = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) prio[vb + i] = mg;
+  if (threadIdx.x < 3) {
+    sh.cnt[threadIdx.x] = sh.hcnt[threadIdx.x] = 0;
+    sh.mn[threadIdx.x] = 0xFFFFFFFFu;
   }
   __syncthreads();
-  uint32_t priority = 0;
-  int last_level = -1;
-  while (sh.todo > 0) {
-    const int level = sh.level;
-    __syncthreads();
+  int head = 0, level = 0, last_level = 0;  // order[0, head) has been processed
+  uint32_t priority = 0, ph = 0;            // ph: this phase's slot
+  auto next_phase = [&]() { ph = ph == 2 ? 0 : ph + 1; };
+  auto reset_next = [&]() {
     if (threadIdx.x == 0) {
-      sh.fcnt = 0;
-      sh.minv = INT_MAX;
+      const uint32_t q = ph == 2 ? 0 : ph + 1;
+      sh.cnt[q] = sh.hcnt[q] = 0;
+      sh.mn[q] = 0xFFFFFFFFu;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      if (score[i] == -1) {
-        const int d = sdeg_get(sdeg, i);
-        if (d <= level) {  // == level: a remaining vertex never has less
-          score[i] = (int16_t)level;
-          F0[atomicAdd(&sh.fcnt, 1)] = i;
-        } else {
-          atomicMin(&sh.minv, d);
-        }
+  };
+  while (head < n) {
+    // scan: the remaining vertices of degree `level` are the level's first round
+    reset_next();
+    uint32_t mn = 0xFFFFFFFFu;
+    for (int k0 = 32 * w; k0 < words; k0 += 32 * nw) {
+      const int k = k0 + lane;
+      const uint32_t x = k < words ? sdeg[k] : 0xFFFFFFFFu;
+      const uint32_t d0 = x & 0xFFFFu, d1 = x >> 16;
+      // == level: a remaining vertex never has less
+      const bool t0 = d0 < SEG_GONE && d0 <= (uint32_t)level;
+      const bool t1 = d1 < SEG_GONE && d1 <= (uint32_t)level;
+      if (!t0 && d0 < SEG_GONE) mn = min(mn, d0);
+      if (!t1 && d1 < SEG_GONE) mn = min(mn, d1);
+      const uint32_t m0 = __ballot_sync(MCE_FULL, t0), m1 = __ballot_sync(MCE_FULL, t1);
+      if (m0 | m1) {
+        if (t0 || t1) sdeg[k] = x | (t0 ? SEG_GONE : 0u) | (t1 ? SEG_GONE << 16 : 0u);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(&sh.cnt[ph], (uint32_t)(__popc(m0) + __popc(m1)));
+        base = __shfl_sync(MCE_FULL, base, 0) + (uint32_t)head;
+        if (t0) order[base + __popc(m0 & lt)] = (uint16_t)(2 * k);
+        if (t1) order[base + __popc(m0) + __popc(m1 & lt)] = (uint16_t)(2 * k + 1);
       }
     }
+    mn = __reduce_min_sync(MCE_FULL, mn);
+    if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(&sh.mn[ph], mn);
     __syncthreads();
-    if (sh.fcnt == 0) {  // no vertex at this level: go to the lowest remaining degree
-      __syncthreads();
-      if (threadIdx.x == 0) sh.level = sh.minv;
-      __syncthreads();
+    int cnt = (int)sh.cnt[ph];
+    const uint32_t lowest = sh.mn[ph];
+    next_phase();
+    if (cnt == 0) {  // no vertex at this level: go to the lowest remaining degree
+      if (lowest == 0xFFFFFFFFu) break;
+      level = (int)lowest;
       continue;
     }
-    int32_t *F = F0, *Gq = G0;
-    for (;;) {
-      const int cnt = sh.fcnt;
-      __syncthreads();
-      if (cnt == 0) break;
-      last_level = level;
-      if (threadIdx.x == 0) {
-        sh.todo -= cnt;
-        sh.ncnt = 0;
+    last_level = level;
+    while (cnt > 0) {
+      reset_next();
+      const int end = head + cnt;  // this round's slice; the next one's begins here
+      const bool last = end >= n;  // the final round keeps priority m_g
+      for (int i = head + (int)threadIdx.x; i < end; i += blockDim.x) {
+        const int v = order[i];
+        core[vb + v] = level;
+        if (!last) prio[vb + v] = priority;
       }
-      __syncthreads();
-      if (sh.todo == 0) break;  // the final round keeps priority m_g
-      for (int i = threadIdx.x; i < cnt; i += blockDim.x) prio[vb + F[i]] = priority;
-      for (int i = w; i < cnt; i += nw) {
-        const int64_t v = vb + F[i];
-        for (int32_t j = rp[v] + lane; j < rp[v + 1]; j += 32) {
-          const int u = (int)(col[j] - vb);
-          if ((unsigned)u >= (unsigned)n) continue;  // not this graph's vertex (invalid input)
-          if (*(volatile int16_t *)&score[u] == -1) {
-            const int old = sdeg_dec(sdeg, u);
-            if (old == level + 1) {
-              score[u] = (int16_t)level;
-              Gq[atomicAdd(&sh.ncnt, 1)] = u;
+      if (last) {
+        head = end;
+        break;
+      }
+      // lower the degree of neighbour c (in: this lane has one); a vertex whose
+      // degree falls to `level` joins the next round
+      auto lower = [&](bool in, int32_t c) {
+        const uint32_t u = (uint32_t)(c - (int32_t)vb);
+        bool p = false;
+        if (in && u < (uint32_t)n) {  // else: not this graph's vertex (invalid input)
+          const uint32_t s = (u & 1u) * 16u;
+          p = ((atomicSub(&sdeg[u >> 1], 1u << s) >> s) & 0xFFFFu) == (uint32_t)level + 1u;
+          if (p) atomicOr(&sdeg[u >> 1], SEG_GONE << s);
+        }
+        const uint32_t mask = __ballot_sync(MCE_FULL, p);
+        if (mask) {
+          uint32_t base = 0;
+          if (lane == 0) base = atomicAdd(&sh.cnt[ph], (uint32_t)__popc(mask));
+          base = __shfl_sync(MCE_FULL, base, 0) + (uint32_t)(end + __popc(mask & lt));
+          if (p && base < (uint32_t)n) order[base] = (uint16_t)u;
+        }
+      };
+      const int g = min(SEG_GROUP, (cnt + nw - 1) / nw);  // spread small rounds over the warps
+      for (int i0 = head + w * g; i0 < end; i0 += nw * g) {
+        const int rows = min(g, end - i0);
+        int32_t b = 0, e = 0;
+        if (lane < rows) {
+          const int v = order[i0 + lane];
+          b = rp[vb + v];
+          e = rp[vb + v + 1];
+          if (e - b > SEG_HEAVY) {
+            const uint32_t hp = atomicAdd(&sh.hcnt[ph], 1u);
+            if (hp < (uint32_t)SEG_HEAVY_MAX) {
+              sh.heavy[hp] = (uint16_t)v;
+              e = b;
             }
+          }
+        }
+        int32_t U[SEG_GROUP];
+#pragma unroll
+        for (int k = 0; k < SEG_GROUP; ++k) {  // every row's first window
+          const int32_t j = __shfl_sync(MCE_FULL, b, k) + lane;
+          const bool in = k < rows && j < __shfl_sync(MCE_FULL, e, k);
+          U[k] = in ? col[j] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < SEG_GROUP; ++k)
+          if (k < rows) lower(U[k] >= 0, U[k]);
+        for (uint32_t lm = __ballot_sync(MCE_FULL, e - b > 32); lm; lm &= lm - 1) {
+          const int k = __ffs(lm) - 1;  // the rest of rows longer than a window
+          const int32_t bk = __shfl_sync(MCE_FULL, b, k), ek = __shfl_sync(MCE_FULL, e, k);
+          for (int32_t j0 = bk + 32; j0 < ek; j0 += 128) {
+            int32_t c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) c[q] = j0 + 32 * q + lane < ek ? col[j0 + 32 * q + lane] : -1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (j0 + 32 * q < ek) lower(c[q] >= 0, c[q]);
           }
         }
       }
       __syncthreads();
-      if (threadIdx.x == 0) sh.fcnt = sh.ncnt;
-      int32_t *t = F;
-      F = Gq;
-      Gq = t;
+      const int hc = min((int)sh.hcnt[ph], SEG_HEAVY_MAX);
+      if (hc > 0) {
+        for (int h = 0; h < hc; ++h) {
+          const int64_t v = vb + sh.heavy[h];
+          const int32_t bk = rp[v], ek = rp[v + 1];
+          for (int32_t j0 = bk + 32 * w; j0 < ek; j0 += 32 * nw) {
+            const int32_t c = j0 + lane < ek ? col[j0 + lane] : -1;
+            lower(c >= 0, c);
+          }
+        }
+        __syncthreads();
+      }
+      head = end;
+      cnt = min((int)sh.cnt[ph], n - head);
+      next_phase();
       ++priority;
-      __syncthreads();
     }
-    if (threadIdx.x == 0) sh.level = level + 1;
-    __syncthreads();
+    ++level;
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) core[vb + i] = score[i];
   if (threadIdx.x == 0) {
     atomicMax(&ctl->rounds, priority);
-    atomicMax(&ctl->degeneracy, last_level < 0 ? 0 : last_level);
+    atomicMax(&ctl->degeneracy, last_level);
   }
   __syncthreads();
+}
+
+// A single graph of at most SEG_SMEM_N vertices and PEEL_ONE_M arcs: one
+// block, whose rounds cost a block barrier each instead of a grid barrier.
+constexpr int PEEL_ONE_BLOCK = 1024;
+constexpr int64_t PEEL_ONE_M = 1 << 22;
+__global__ void __launch_bounds__(PEEL_ONE_BLOCK)
+    peel_one_kernel(int n, uint32_t m, const int32_t *__restrict__ rp,
+                    const int32_t *__restrict__ col, int32_t *core, uint32_t *prio, PeelCtl *ctl) {
+  __shared__ SegShared sh;
+  extern __shared__ uint32_t seg_dyn[];
+  const int n2 = (n + 1) & ~1;
+  peel_graph_smem(rp, col, core, prio, 0, n, m, seg_dyn, (uint16_t *)(seg_dyn + n2 / 2), sh, ctl);
 }
 
 __global__ void __launch_bounds__(SEG_BLOCK)
@@ -603,9 +690,9 @@ __global__ void __launch_bounds__(SEG_BLOCK)
                          const int32_t *__restrict__ order, int32_t G, PeelCtl *ctl,
                          uint32_t *next, int smem_n) {
   __shared__ SegShared sh;
-  extern __shared__ uint32_t seg_dyn[];  // smem_n / 2 degree words, then smem_n cores
+  extern __shared__ uint32_t seg_dyn[];  // smem_n / 2 degree words, then smem_n ids
   uint32_t *sdeg = seg_dyn;
-  int16_t *score = (int16_t *)(seg_dyn + smem_n / 2);
+  uint16_t *vord = (uint16_t *)(seg_dyn + smem_n / 2);
   const int lane = (int)lane_id(), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (;;) {
     if (threadIdx.x == 0) sh.g = atomicAdd(next, 1u);  // next graph, largest first
@@ -616,7 +703,7 @@ __global__ void __launch_bounds__(SEG_BLOCK)
     const int64_t vb = vtx_off[gr] - gr, n = vtx_off[gr + 1] - vtx_off[gr] - 1;
     const uint32_t mg = (uint32_t)(arc_off[gr + 1] - arc_off[gr]);
     if (n <= smem_n) {
-      peel_graph_smem(rp, col, core, prio, fa + vb, fb + vb, vb, (int)n, mg, sdeg, score, sh, ctl);
+      peel_graph_smem(rp, col, core, prio, vb, (int)n, mg, sdeg, vord, sh, ctl);
       continue;
     }
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -732,7 +819,7 @@ int peel_segments_launch(const PeelArgs &a, const int64_t *vtx_off, const int64_
                     cudaStream_t st) -> int {
     if (cnt <= 0) return MCE_OK;
     const int smem_n = nmax <= 0 ? 0 : (int)((std::min<int64_t>(nmax, SEG_SMEM_N) + 1) & ~1);
-    const size_t smem = (size_t)smem_n * 4;  // 2 bytes of degree + 2 of core per vertex
+    const size_t smem = (size_t)smem_n * 4;  // 2 bytes of degree + 2 of order per vertex
     int per_sm = 0;
     MCE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, peel_segments_kernel, threads,
                                                            smem));
@@ -776,6 +863,18 @@ size_t peel_ctl_bytes() { return sizeof(PeelCtl); }
 
 int peel_launch(const PeelArgs &a, cudaStream_t s, int *launches) {
   int dev = 0, sms = 0, per_sm = 0, coop = 0;
+  if (a.n <= SEG_SMEM_N && a.m <= PEEL_ONE_M && a.solo_max == 0) {
+    const size_t smem = (size_t)((a.n + 1) & ~(int64_t)1) * 4;
+    // set on every call: the attribute belongs to the current device
+    MCE_CUDA(cudaFuncSetAttribute(peel_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  SEG_SMEM_N * 4));
+    MCE_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(PeelCtl), s));
+    peel_one_kernel<<<1, PEEL_ONE_BLOCK, smem, s>>>((int)a.n, (uint32_t)a.m, a.rp, a.col, a.core,
+                                                    a.prio, (PeelCtl *)a.ctl);
+    MCE_CUDA(cudaGetLastError());
+    if (launches) *launches += 1;
+    return MCE_OK;
+  }
   MCE_CUDA(cudaGetDevice(&dev));
   MCE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   MCE_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
