@@ -50,57 +50,16 @@ __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void red_release(uint32_t *p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) {
   return *(const volatile uint32_t *)p;
 }
 
 __device__ __forceinline__ unsigned long long ld_volatile(const unsigned long long *p) {
   return *(const volatile unsigned long long *)p;
-}
-
-// Grid-wide barrier for a kernel whose blocks are all resident (launched with
-// cudaLaunchCooperativeKernel, which refuses a grid that cannot be).  Bounded:
-// if the other blocks do not arrive within `limit_ns`, the flag `err` gets
-// MCE_ERR_WAIT_TIMEOUT and the function returns false so the caller can stop.
-struct GridBarrier {
-  uint32_t count;
-  uint32_t gen;
-};
-
-__device__ __forceinline__ bool grid_sync(GridBarrier *b, uint32_t nblocks, uint32_t *err,
-                                          uint64_t limit_ns) {
-  __syncthreads();
-  __shared__ uint32_t ok;
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const uint32_t g = ld_volatile(&b->gen);
-    __threadfence();
-    const uint32_t arrived = atomicAdd(&b->count, 1u);
-    if (arrived == nblocks - 1) {
-      atomicExch(&b->count, 0u);
-      __threadfence();
-      atomicAdd(&b->gen, 1u);
-    } else {
-      const uint64_t t0 = globaltimer_ns();
-      uint32_t ns = 32;
-      while (ld_volatile(&b->gen) == g) {
-        if (ld_volatile(err) & MCE_ERR_WAIT_TIMEOUT) {
-          ok = 0;
-          break;
-        }
-        if (globaltimer_ns() - t0 > limit_ns) {
-          atomicOr(err, MCE_ERR_WAIT_TIMEOUT);
-          ok = 0;
-          break;
-        }
-        __nanosleep(ns);
-        if (ns < 256) ns <<= 1;
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok != 0;
 }
 
 // ---- 1-D bulk copies global -> shared through an mbarrier (the TMA unit's

@@ -18,8 +18,11 @@
 //  - a level with no vertex of degree k runs no round (the scan below jumps
 //    straight to the smallest remaining degree, which numbers rounds the
 //    same way).
-// Decrements of a vertex that is already removed or queued are skipped;
-// they cannot change any round's membership.
+// Decrements of a vertex that is already removed or queued change no round's
+// membership: its degree is at most its level and only falls, while a vertex
+// joins a round only when its degree falls from level + 1.  So no core number
+// is read before a decrement, and a scan tells the remaining vertices by
+// their degree alone.
 #include <climits>
 
 #include <cooperative_groups.h>
@@ -32,7 +35,7 @@
 namespace mce {
 
 struct PeelCtl {
-  GridBarrier bar;
+  uint32_t arrived;    // blocks that reached a phase barrier so far, over all phases
   uint32_t err;
   uint32_t fcnt[3];    // light frontier sizes, one slot per phase mod 3
   unsigned long long hpack[3];  // heavy frontier: (count << 32) | 32-edge chunks
@@ -57,7 +60,13 @@ struct PeelCtl {
 
 namespace {
 
-constexpr int PEEL_BLOCK = 512;
+// One block per SM: a phase costs one arrival per block at the barrier.  The
+// grid-wide peel is bounded by the latency of its phases (a barrier, then some
+// six dependent accesses); with one counter that only grows, one reader of the
+// phase's counters per block and no core number read before a decrement, a
+// round of BA n = 1e6 takes 10 us instead of 17 (peel 3.1 -> 1.77 ms) and the
+// order of R-MAT 17 3.1 ms instead of 6.4.
+constexpr int PEEL_BLOCK = 1024;
 // A frontier of at most solo_max vertices is peeled by block 0 alone, round
 // after round with __syncthreads between them, for up to SOLO_ROUNDS rounds
 // (well inside the other blocks' barrier wait limit).
@@ -150,35 +159,80 @@ __device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long 
   return *(const volatile unsigned long long *)p;
 }
 
-__device__ __forceinline__ uint32_t frontier_size(const PeelCtl *ctl, int slot) {
-  return ld_volatile(&ctl->fcnt[slot]) + (uint32_t)(ld_volatile64(&ctl->hpack[slot]) >> 32);
+// What a phase left behind, read by one thread per block (thousands of warps
+// reading the same few words would queue at one L2 slice).
+struct PhaseOut {
+  uint32_t light, heavy, chunks;  // the frontier: light and heavy vertices, 32-edge chunks
+  uint32_t alive, lowest;         // a scan's survivors and their lowest degree
+  uint32_t ok;
+};
+
+__device__ __forceinline__ void read_frontier(const PeelCtl *ctl, uint32_t slot, PhaseOut &o) {
+  const unsigned long long hp = ld_volatile64(&ctl->hpack[slot]);
+  o.light = ld_volatile(&ctl->fcnt[slot]);
+  o.heavy = (uint32_t)(hp >> 32);
+  o.chunks = (uint32_t)hp;
+}
+
+// Grid barrier at the end of a phase (all blocks are resident: cooperative
+// launch) and the counters of its output: frontier slot q, alive slot s.  One
+// counter that only grows, one release add per block and one acquiring reader
+// per block; bounded: false (and MCE_ERR_WAIT_TIMEOUT) after limit_ns.
+__device__ __forceinline__ bool phase_sync(PeelCtl *ctl, uint32_t nblocks, uint32_t &target,
+                                           uint32_t q, uint32_t s, PhaseOut &out,
+                                           uint64_t limit_ns) {
+  __syncthreads();
+  target += nblocks;
+  if (threadIdx.x == 0) {
+    red_release(&ctl->arrived, 1u);
+    uint32_t ok = 1, spins = 0;
+    uint64_t t0 = 0;
+    while ((int32_t)(ld_acquire(&ctl->arrived) - target) < 0) {
+      if ((++spins & 255u) == 0) {
+        const uint64_t now = globaltimer_ns();
+        if (!t0) t0 = now;
+        if (ld_volatile(&ctl->err) & MCE_ERR_WAIT_TIMEOUT) {
+          ok = 0;
+          break;
+        }
+        if (now - t0 > limit_ns) {
+          atomicOr(&ctl->err, MCE_ERR_WAIT_TIMEOUT);
+          ok = 0;
+          break;
+        }
+      }
+    }
+    read_frontier(ctl, q, out);
+    out.alive = ld_volatile(&ctl->acnt[s]);
+    out.lowest = ld_volatile(&ctl->amin[s]);
+    out.ok = ok;
+  }
+  __syncthreads();
+  return out.ok != 0;
 }
 
 // Lower the degree of neighbour col[j] of a vertex being removed; true if it
 // falls to `level` (it then joins the next round).
 __device__ __forceinline__ bool peel_edge(int32_t j, int32_t e, int32_t level,
                                           const int32_t *__restrict__ col, int32_t *deg,
-                                          int32_t *core, int32_t &u) {
+                                          int32_t &u) {
   u = 0;
   if (j >= e) return false;
   u = col[j];
-  if (ld_volatile((const uint32_t *)&core[u]) != 0xFFFFFFFFu) return false;
-  const int32_t old = atomicSub(&deg[u], 1);
-  if (old != level + 1) return false;
-  core[u] = level;
-  return true;
+  return atomicSub(&deg[u], 1) == level + 1;
 }
 
-// One peel round (phase q) over the frontier in slot q % 3, executed by the
-// threads [t0, t0 + nt) (the whole grid, or block 0 alone): set the round's
-// priority, lower the neighbours' degrees and append every neighbour whose
-// degree falls to `level` to the frontier in slot (q + 1) % 3.
-__device__ __forceinline__ void peel_round(uint32_t q, int32_t level, uint32_t priority,
-                                           int64_t t0, int64_t nt, int64_t cap,
-                                           const int32_t *__restrict__ rp,
-                                           const int32_t *__restrict__ col, int32_t *deg,
-                                           int32_t *core, uint32_t *prio, int32_t *const *fr,
-                                           int32_t *const *hb, PeelCtl *ctl, int32_t *stage) {
+// One peel round (phase q) over the frontier in slot q % 3 (its counters in
+// `in`), executed by the threads [t0, t0 + nt) (the whole grid, or block 0
+// alone): set the round's priority, lower the neighbours' degrees and append
+// every neighbour whose degree falls to `level` to the frontier in slot
+// (q + 1) % 3.
+__device__ __noinline__ void peel_round(uint32_t q, int32_t level, uint32_t priority,
+                                        const PhaseOut &in, int64_t t0, int64_t nt, int64_t cap,
+                                        const int32_t *__restrict__ rp,
+                                        const int32_t *__restrict__ col, int32_t *deg,
+                                        int32_t *core, uint32_t *prio, int32_t *const *fr,
+                                        int32_t *const *hb, PeelCtl *ctl, int32_t *stage) {
   const uint32_t lane = lane_id();
   Stage st{stage, 0};
   const int fn = (q + 1) % 3;
@@ -186,13 +240,14 @@ __device__ __forceinline__ void peel_round(uint32_t q, int32_t level, uint32_t p
     ctl->fcnt[(q + 2) % 3] = 0;
     ctl->hpack[(q + 2) % 3] = 0;
   }
-  const uint32_t lc = ld_volatile(&ctl->fcnt[q % 3]);
-  const unsigned long long hp = ld_volatile64(&ctl->hpack[q % 3]);
-  const uint32_t hc = (uint32_t)(hp >> 32), hch = (uint32_t)hp;
+  const uint32_t lc = in.light, hc = in.heavy, hch = in.chunks;
   const int32_t *Fc = fr[q % 3], *HB = hb[q % 3];
   int32_t *Fn = fr[fn], *HBn = hb[fn];
-  for (int64_t i = t0; i < lc; i += nt) prio[Fc[i]] = priority;
-  for (int64_t i = t0; i < hc; i += nt) prio[Fc[cap - 1 - i]] = priority;
+  for (int64_t i = t0; i < (int64_t)lc + hc; i += nt) {
+    const int32_t v = i < lc ? Fc[i] : Fc[cap - 1 - (i - lc)];
+    prio[v] = priority;
+    core[v] = level;
+  }
   auto push = [&](bool p, int32_t u) {
     int32_t du = 0;
     if (p) du = rp[u + 1] - rp[u];
@@ -226,23 +281,18 @@ __device__ __forceinline__ void peel_round(uint32_t q, int32_t level, uint32_t p
         U[k] = in ? col[j] : 0;
         live[k] = in;
       }
-#pragma unroll
-      for (int k = 0; k < R; ++k)
-        live[k] = live[k] && ld_volatile((const uint32_t *)&core[U[k]]) == 0xFFFFFFFFu;
       int32_t old[R];
 #pragma unroll
       for (int k = 0; k < R; ++k) old[k] = live[k] ? atomicSub(&deg[U[k]], 1) : 0;
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        const bool p = live[k] && old[k] == level + 1;
-        if (p) core[U[k]] = level;
-        push(p, U[k]);
+        push(live[k] && old[k] == level + 1, U[k]);
       }
       for (int k = 0; k < rows; ++k) {  // the rest of rows longer than a window
         const int32_t bk = __shfl_sync(MCE_FULL, b, k), ek = __shfl_sync(MCE_FULL, e, k);
         for (int32_t j0 = bk + 32; j0 < ek; j0 += 32) {
           int32_t u;
-          const bool p = peel_edge(j0 + (int32_t)lane, ek, level, col, deg, core, u);
+          const bool p = peel_edge(j0 + (int32_t)lane, ek, level, col, deg, u);
           push(p, u);
         }
       }
@@ -253,7 +303,7 @@ __device__ __forceinline__ void peel_round(uint32_t q, int32_t level, uint32_t p
       const int32_t b = rp[v], e = rp[v + 1];
       for (int32_t j0 = b; j0 < e; j0 += 32) {
         int32_t u;
-        const bool p = peel_edge(j0 + (int32_t)lane, e, level, col, deg, core, u);
+        const bool p = peel_edge(j0 + (int32_t)lane, e, level, col, deg, u);
         push(p, u);
       }
     }
@@ -273,7 +323,7 @@ __device__ __forceinline__ void peel_round(uint32_t q, int32_t level, uint32_t p
     const int32_t e = rp[v + 1];
     const int32_t j = rp[v] + ((int32_t)c - HB[h]) * 32 + (int32_t)lane;
     int32_t u;
-    const bool p = peel_edge(j, e, level, col, deg, core, u);
+    const bool p = peel_edge(j, e, level, col, deg, u);
     push(p, u);
   }
   stage_flush(st, Fn, &ctl->fcnt[fn]);
@@ -286,6 +336,7 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
                 int32_t *front2, int32_t *hb0, int32_t *hb1, int32_t *hb2, PeelCtl *ctl,
                 uint64_t limit_ns, uint32_t solo_max) {
   __shared__ int32_t stage_all[PEEL_BLOCK / 32][STAGE];
+  __shared__ PhaseOut out;  // of the latest phase
   int32_t *const stage = stage_all[threadIdx.x >> 5];
   const uint32_t nblocks = gridDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -308,7 +359,8 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
     ctl->acnt[1] = ctl->acnt[2] = 0;
     ctl->amin[0] = ctl->amin[1] = ctl->amin[2] = 0xFFFFFFFFu;
   }
-  if (!grid_sync(&ctl->bar, nblocks, &ctl->err, limit_ns)) return;
+  uint32_t target = 0;  // arrivals at the end of the current phase
+  if (!phase_sync(ctl, nblocks, target, 0, 0, out, limit_ns)) return;
 
   // phase timers of block 0 (diagnostics only)
   unsigned long long t_ts = 0, t_tr = 0, t_w = 0, mark = tid == 0 ? globaltimer_ns() : 0;
@@ -332,7 +384,7 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
   uint32_t q = 0, s = 0;
   while (todo > 0) {
     // ---- scan: split the alive list into {deg == level} and {deg > level}
-    const uint32_t nalive = ld_volatile(&ctl->acnt[s % 3]);
+    const uint32_t nalive = out.alive;
     const int32_t *A = alist[s & 1];
     int32_t *A2 = alist[(s + 1) & 1];
     const int fo = (q + 1) % 3, ao = (s + 1) % 3;
@@ -354,12 +406,11 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
         bool live = false;
         if (i < nalive) {
           v = A[i];
-          live = ld_volatile((const uint32_t *)&core[v]) == 0xFFFFFFFFu;
+          live = true;
           d = deg[v];
         }
         const bool inF = live && d == level;
         const bool keep = live && d > level;
-        if (inF) core[v] = level;
         const int32_t dv = inF ? rp[v + 1] - rp[v] : 0;
         const bool heavy = inF && dv > HEAVY_DEG;
         block_append2(inF && !heavy, v, F, &ctl->fcnt[fo], keep, v, A2, &ctl->acnt[ao]);
@@ -370,15 +421,15 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
       if (lane == 0 && mymin != 0xFFFFFFFFu) atomicMin(&ctl->amin[ao], mymin);
     }
     tick(t_ts);
-    if (!grid_sync(&ctl->bar, nblocks, &ctl->err, limit_ns)) return;
-    tick(t_w);
     ++q;
     ++s;
-    uint32_t cnt = frontier_size(ctl, q % 3);
+    if (!phase_sync(ctl, nblocks, target, q % 3, s % 3, out, limit_ns)) return;
+    tick(t_w);
+    uint32_t cnt = out.light + out.heavy;
     if (cnt == 0) {
       // no vertex of degree `level` remains: jump to the smallest degree
       // (a rescan at that level always finds the vertex that attains it)
-      const uint32_t mn = ld_volatile(&ctl->amin[s % 3]);
+      const uint32_t mn = out.lowest;
       if (mn == 0xFFFFFFFFu || (int32_t)mn <= level) {
         if (tid == 0) atomicOr(&ctl->err, MCE_ERR_QUEUE);  // inconsistent state: stop
         break;
@@ -391,27 +442,39 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
     while (cnt > 0) {
       degen = level;
       todo -= cnt;
-      if (todo == 0) break;  // the final round keeps priority = m
+      if (todo == 0) {  // the final round keeps priority = m
+        const int32_t *Fc = fr[q % 3];
+        for (int64_t i = tid; i < (int64_t)out.light + out.heavy; i += nthr)
+          core[i < out.light ? Fc[i] : Fc[n - (i - out.light)]] = level;
+        break;
+      }
       if (cnt <= solo_max) {
         // Small frontier: block 0 peels consecutive rounds alone.  The first
         // barrier lets every block read `cnt` before block 0 recycles slots.
         tick(t_tr);
-        if (!grid_sync(&ctl->bar, nblocks, &ctl->err, limit_ns)) return;
+        if (!phase_sync(ctl, nblocks, target, q % 3, s % 3, out, limit_ns)) return;
         tick(t_w);
         if (blockIdx.x == 0) {
           uint32_t it = 0;
           for (;;) {
-            peel_round(q, level, priority, threadIdx.x, blockDim.x, (int64_t)n + 1, rp, col,
+            peel_round(q, level, priority, out, threadIdx.x, blockDim.x, (int64_t)n + 1, rp, col,
                        deg, core, prio, fr, hb, ctl, stage);
             __syncthreads();
             ++q;
-            cnt = frontier_size(ctl, q % 3);
+            if (threadIdx.x == 0) read_frontier(ctl, q % 3, out);
+            __syncthreads();
+            cnt = out.light + out.heavy;
             ++priority;
             ++rounds;
             if (cnt == 0 || cnt > solo_max || ++it >= SOLO_ROUNDS) break;  // cnt not yet counted
             degen = level;
             todo -= cnt;
-            if (todo == 0) break;  // the final round keeps priority = m
+            if (todo == 0) {  // the final round keeps priority = m
+              const int32_t *Fc = fr[q % 3];
+              for (int64_t i = threadIdx.x; i < (int64_t)cnt; i += blockDim.x)
+                core[i < out.light ? Fc[i] : Fc[n - (i - out.light)]] = level;
+              break;
+            }
             __syncthreads();       // every thread has read cnt before slots rotate
           }
           if (threadIdx.x == 0) {
@@ -425,10 +488,13 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
           }
         }
         tick(t_tr);
-        if (!grid_sync(&ctl->bar, nblocks, &ctl->err, limit_ns)) return;
+        if (!phase_sync(ctl, nblocks, target, q % 3, s % 3, out, limit_ns)) return;
         tick(t_w);
         q = ld_volatile(&ctl->solo_q);
         cnt = ld_volatile(&ctl->solo_cnt);
+        __syncthreads();  // every thread is past the barrier's output
+        if (threadIdx.x == 0) read_frontier(ctl, q % 3, out);
+        __syncthreads();
         priority = ld_volatile(&ctl->solo_priority);
         rounds = ld_volatile(&ctl->solo_rounds);
         todo = *(volatile int64_t *)&ctl->solo_todo;
@@ -436,13 +502,13 @@ __global__ void __launch_bounds__(PEEL_BLOCK)
         if (todo == 0) break;
         continue;
       }
-      peel_round(q, level, priority, tid, nthr, (int64_t)n + 1, rp, col, deg, core, prio, fr, hb,
-                 ctl, stage);
+      peel_round(q, level, priority, out, tid, nthr, (int64_t)n + 1, rp, col, deg, core, prio, fr,
+                 hb, ctl, stage);
       tick(t_tr);
-      if (!grid_sync(&ctl->bar, nblocks, &ctl->err, limit_ns)) return;
-      tick(t_w);
       ++q;
-      cnt = frontier_size(ctl, q % 3);
+      if (!phase_sync(ctl, nblocks, target, q % 3, s % 3, out, limit_ns)) return;
+      tick(t_w);
+      cnt = out.light + out.heavy;
       ++priority;
       ++rounds;
     }
@@ -672,8 +738,13 @@ __device__ void peel_graph_smem(const int32_t *__restrict__ rp, const int32_t *_
 
 // A single graph of at most SEG_SMEM_N vertices and PEEL_ONE_M arcs: one
 // block, whose rounds cost a block barrier each instead of a grid barrier.
+// One block against the grid: ER n = 200, 1,000 and 10,000 (degree 10 to 20)
+// 0.027, 0.053 and 0.195 ms against 0.094, 0.231 and 0.251; ER n = 16,384 of
+// 492 k and 982 k arcs 0.383 and 0.494 against 0.329 and 0.400; with many
+// rounds (R-MAT 13 of 204 k arcs, BA of 1.02 M) 0.437 and 0.941 against 1.359
+// and 1.528: the limit lies between.
 constexpr int PEEL_ONE_BLOCK = 1024;
-constexpr int64_t PEEL_ONE_M = 1 << 22;
+constexpr int64_t PEEL_ONE_M = 1 << 19;
 __global__ void __launch_bounds__(PEEL_ONE_BLOCK)
     peel_one_kernel(int n, uint32_t m, const int32_t *__restrict__ rp,
                     const int32_t *__restrict__ col, int32_t *core, uint32_t *prio, PeelCtl *ctl) {
@@ -881,7 +952,7 @@ int peel_launch(const PeelArgs &a, cudaStream_t s, int *launches) {
   if (!coop) return MCE_ENODEV;
   MCE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, peel_kernel, PEEL_BLOCK, 0));
   if (per_sm < 1) return MCE_ECUDA;
-  per_sm = per_sm > 2 ? 2 : per_sm;
+  per_sm = 1;
   int32_t n = (int32_t)a.n;
   uint32_t m = (uint32_t)a.m;
   PeelCtl *ctl = (PeelCtl *)a.ctl;

@@ -31,7 +31,8 @@ def hubs(n, k, seed):
     ("16,384 vertices", lambda: mce.gen_ba(16384, 8, 5, 10, 20, 60)),
     ("16,385 vertices: grid", lambda: mce.gen_er(16385, 9.0 / 16385, 6)),
     ("R-MAT core", lambda: mce.gen_rmat(13, 16, 0.57, 0.19, 0.19, 3)),
-    ("just above the arc limit: grid", lambda: mce.gen_er(3000, 0.47, 8)),
+    ("just above the arc limit: grid", lambda: mce.gen_er(3000, 0.06, 8)),
+    ("grid, many rounds and long rows", lambda: mce.gen_rmat(15, 12, 0.57, 0.19, 0.19, 4)),
 ], ids=lambda x: x if isinstance(x, str) else "")
 def test_peel_matches_oracle(name, make):
     g = make()
