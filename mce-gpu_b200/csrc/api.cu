@@ -123,6 +123,8 @@ namespace {
 constexpr uint64_t WAIT_LIMIT_NS = 20ull * 1000 * 1000 * 1000;  // 20 s per barrier wait
 constexpr uint64_t IDLE_LIMIT_NS = 30ull * 1000 * 1000 * 1000;  // 30 s without any progress
 constexpr uint32_t QUEUE_CAP = 1u << 14;                        // tasks per class queue
+constexpr size_t QUEUE_HDR = 512;                               // bytes before its slots
+static_assert(sizeof(QueueHdr) <= QUEUE_HDR, "queue header");
 constexpr int DEFAULT_DONATE_MIN = 10;
 constexpr int64_t BATCH_PART_MIN_ARCS = 1 << 20;  // mce_batch_count_host: smaller batches in one part
 constexpr uint32_t DEFAULT_SOLO_MAX = 0;     // measured slower than grid-wide rounds
@@ -446,7 +448,7 @@ int read_shape(mce_graph *g, cudaStream_t s) {
 
 // Queue of class c laid out in one buffer: header | seq[cap] | payload.
 int ensure_queue(mce_graph *g, int c, uint32_t words, QueueView *out) {
-  const size_t hdr = 256, seq = (size_t)QUEUE_CAP * 4;
+  const size_t hdr = QUEUE_HDR, seq = (size_t)QUEUE_CAP * 4;
   const size_t need = hdr + seq + (size_t)QUEUE_CAP * words * 8;
   if (need > g->qbytes[c]) {
     dfree(g->qbuf[c]);
@@ -1288,7 +1290,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     }
     if (share_q) {
       const uint32_t words = bk_task_words(c, dcap);
-      const size_t qneed = 256 + (size_t)QUEUE_CAP * 4 + (size_t)QUEUE_CAP * words * 8;
+      const size_t qneed = QUEUE_HDR + (size_t)QUEUE_CAP * 4 + (size_t)QUEUE_CAP * words * 8;
       if (qneed > g->qbytes[c] && g->qbuf[c]) {  // ensure_queue would free it in use
         retired.push_back(g->qbuf[c]);
         g->qbuf[c] = nullptr;

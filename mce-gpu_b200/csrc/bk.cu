@@ -114,10 +114,7 @@ __global__ void __launch_bounds__(REG_BLOCK, (NR == 1 && sizeof(Word) == 4) ? 6 
     }
   }
   if (share) {
-    if (lane == 0) {
-      atomicSub(&a.q.hdr->work, 1u);
-      atomicAdd(&a.q.hdr->epoch, 1u);
-    }
+    root_phase_done(a.q);
     u64 t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
     MCE_BD(BD_QUEUE);
     idle_phase(
@@ -235,10 +232,7 @@ __global__ void __launch_bounds__(MEM_BLOCK, MINB) bk_mem_kernel(BKArgs a, int c
     }
   }
   if (share) {
-    if (lane == 0) {
-      atomicSub(&a.q.hdr->work, 1u);
-      atomicAdd(&a.q.hdr->epoch, 1u);
-    }
+    root_phase_done(a.q);
     const int WM = (a.dcap + 63) >> 6;
     int32_t task_root = -1;
     MCE_BD(BD_QUEUE);

@@ -110,54 +110,56 @@ __device__ __forceinline__ void root_ops_done(const BKArgs &a, int32_t r, u64 op
   if (lane_id() == 0 && a.root_ops && ops) atomicAdd(&a.root_ops[r], ops);
 }
 
+// End of a warp's root phase: it no longer counts as work.
+__device__ __forceinline__ void root_phase_done(const QueueView &q) {
+  if (lane_id() == 0) atomicSub(&q.hdr->work, 1u);
+}
+
 // Idle phase shared by the engines: take tasks until no work is left.
-// `run(words)` processes one task whose words were stored by `put`.
+// put(k, word) receives a task's words, run() processes it.
 template <typename Put, typename Run>
 __device__ void idle_phase(const BKArgs &a, Put put, Run run) {
   const QueueView &q = a.q;
   const uint32_t lane = lane_id();
-  if (lane == 0) atomicAdd(&q.hdr->idle, 1u);
-  uint32_t last_epoch = 0;
-  uint64_t t_last = 0;
-  if (lane == 0) {
-    last_epoch = ld_volatile(&q.hdr->epoch);
-    t_last = globaltimer_ns();
-  }
-  uint32_t ns = 64;
   for (;;) {
-    if (q_pop(q, put)) {
-      if (lane == 0) atomicSub(&q.hdr->idle, 1u);
-      run();
+    uint32_t pos = 0;
+    if (lane == 0) pos = atomicAdd(&q.hdr->head, 1u);
+    pos = __shfl_sync(MCE_FULL, pos, 0);
+    uint32_t last = 0, ns = 64, polls = 0;
+    uint64_t t_last = 0;
+    int state = 0;  // 1: the task is there, 2: nothing left to wait for
+    for (;;) {
       if (lane == 0) {
-        atomicSub(&q.hdr->work, 1u);
-        atomicAdd(&q.hdr->epoch, 1u);
-        atomicAdd(&q.hdr->idle, 1u);
-        t_last = globaltimer_ns();
-      }
-      ns = 64;
-      continue;
-    }
-    int stop = 0;
-    if (lane == 0) {
-      if (ld_volatile(&q.hdr->work) == 0) {
-        stop = 1;
-      } else {
-        const uint32_t e = ld_volatile(&q.hdr->epoch);
-        const uint64_t now = globaltimer_ns();
-        if (e != last_epoch) {
-          last_epoch = e;
-          t_last = now;
-        } else if (now - t_last > a.wait_limit_ns) {
-          atomicOr(a.err, MCE_ERR_WAIT_TIMEOUT);  // no progress anywhere: give up
-          stop = 1;
+        if (q_ready(q, pos)) {
+          state = 1;
+        } else if ((polls++ & 3u) == 0) {
+          const uint32_t work = ld_volatile(&q.hdr->work);
+          if (work == 0) {
+            if (q_leave(q, pos)) state = 2;
+          } else {  // pushes move tail, ends of tasks and root phases move work
+            const uint32_t now_at = ld_volatile(&q.hdr->tail) * 2654435761u + work;
+            const uint64_t now = globaltimer_ns();
+            if (t_last == 0 || now_at != last) {
+              last = now_at;
+              t_last = now;
+            } else if (now - t_last > a.wait_limit_ns) {
+              atomicOr(a.err, MCE_ERR_WAIT_TIMEOUT);  // no progress anywhere: give up
+              q_leave(q, pos);
+              state = 2;
+            }
+          }
         }
       }
+      state = __shfl_sync(MCE_FULL, state, 0);
+      if (state) break;
+      __nanosleep(ns);
+      if (ns < 1024) ns <<= 1;
     }
-    if (__shfl_sync(MCE_FULL, stop, 0)) break;
-    __nanosleep(ns);
-    if (ns < 8192) ns <<= 1;
+    if (state == 2) return;
+    q_take(q, pos, put);
+    run();
+    if (lane == 0) atomicSub(&q.hdr->work, 1u);
   }
-  if (lane == 0) atomicSub(&q.hdr->idle, 1u);
 }
 
 // ---------------------------------------------------------------------------

@@ -7,25 +7,32 @@
 // when every block of the grid sits in the ring, so the whole grid must be
 // resident.  Here the queue holds self-contained tasks - a root and one node
 // of its search tree (P, X and the chosen set as bitmaps over the root's
-// later neighbours) - so any warp can take any task, nobody waits for a
-// particular warp, and termination is a single counter:
+// later neighbours) - so any warp can take any task, and termination is a
+// single counter:
 //   work = warps still in their root phase + tasks queued or running.
-// A warp that has run out of roots takes tasks until work == 0.  Push and
-// pop never block (a full queue means "keep the subtree"); the only wait is
-// an idle warp polling, bounded by a no-progress time limit.
+// A warp that has run out of roots draws a ticket - the ring position of the
+// next task nobody waits for - and polls that position alone, so thousands of
+// idle warps do not meet at one word; donors push while tickets are ahead of
+// tasks, each at a position of its own too (one atomic add).  What bounds the
+// sharing is the chain of dependent accesses from one push to the next: with
+// donors agreeing on the ring's tail by compare-and-swap the device made one
+// push per 0.9 us, and the time of the search of an R-MAT graph of scale 13
+// was its number of pushes.  An idle warp's poll is bounded by a no-progress
+// time limit, a donor's wait for its slot by a count.
 #pragma once
 
 #include "common.cuh"
 
 namespace mce {
 
-struct QueueHdr {
-  uint32_t head, tail;  // ring positions (wrap modulo 2^32)
-  uint32_t work;        // see above
-  uint32_t idle;        // warps polling for a task
-  uint32_t epoch;       // bumped on every push and task completion
-  uint32_t pushed;      // tasks pushed (statistics)
-  uint32_t pad[26];
+struct QueueHdr {  // one word per 128-byte line
+  uint32_t head;   // tickets drawn (ring positions, modulo 2^32) ...
+  uint32_t pad0[31];
+  uint32_t tail;   // ... and tasks pushed
+  uint32_t pad1[31];
+  uint32_t work;   // see above
+  uint32_t pad2[31];
+  uint32_t pushed; // statistics
 };
 
 struct QueueView {
@@ -38,6 +45,10 @@ struct QueueView {
 
 __global__ void queue_init_kernel(QueueView q);
 
+// A ring slot at position pos (modulo cap): seq = pos when empty, pos + 2
+// while a donor writes its task, pos + 1 with the task there, pos + cap once
+// the task was taken - or its ticket given up by a warp that left.
+//
 // Claim a slot and publish `words` task words held by the warp (lane k holds
 // words k, k+32, ...; supplied by `get(k)`).  Returns false if full.
 template <typename Get>
@@ -46,26 +57,23 @@ __device__ __forceinline__ bool q_push(const QueueView &q, Get get) {
   uint32_t pos = 0;
   int ok = 0;
   if (lane == 0) {
-    pos = ld_volatile(&q.hdr->tail);
-    for (int tries = 0; tries < 64; ++tries) {
-      const uint32_t s = ld_acquire(&q.seq[pos & (q.cap - 1)]);
-      const int32_t diff = (int32_t)(s - pos);
-      if (diff == 0) {
-        const uint32_t seen = atomicCAS(&q.hdr->tail, pos, pos + 1);
-        if (seen == pos) {
-          ok = 1;
-          break;
-        }
-        pos = seen;
-      } else if (diff < 0) {
-        break;  // full
-      } else {
-        pos = ld_volatile(&q.hdr->tail);
+    for (int tries = 0; tries < 64 && !ok; ++tries) {
+      pos = atomicAdd(&q.hdr->tail, 1u);
+      uint32_t *s = &q.seq[pos & (q.cap - 1)];
+      uint32_t seen = atomicCAS(s, pos, pos + 2);
+      // a task of the ring's last lap whose taker is still reading it (the ring
+      // is twice as long as there are warps)
+      for (int spin = 0; seen != pos && seen != pos + q.cap && spin < (1 << 20); ++spin) {
+        __nanosleep(64);
+        seen = atomicCAS(s, pos, pos + 2);
       }
-    }
-    if (ok) {
-      atomicAdd(&q.hdr->work, 1u);  // counted before anyone can take it
-      atomicAdd(&q.hdr->pushed, 1u);
+      if (seen == pos) {
+        atomicAdd(&q.hdr->work, 1u);  // counted before anyone can take it
+        atomicAdd(&q.hdr->pushed, 1u);
+        ok = 1;
+      } else if (seen != pos + q.cap) {
+        break;  // the wait ran out: keep the subtree
+      }  // else: a ticket that was given up, try the next position
     }
   }
   ok = __shfl_sync(MCE_FULL, ok, 0);
@@ -77,56 +85,38 @@ __device__ __forceinline__ bool q_push(const QueueView &q, Get get) {
   if (lane == 0) {
     __threadfence();
     st_release(&q.seq[pos & (q.cap - 1)], pos + 1);
-    atomicAdd(&q.hdr->epoch, 1u);
   }
   __syncwarp();
   return true;
 }
 
-// Take a task: on success `put(k, word)` receives every word (lane-strided).
+// Whether the task of ticket `pos` is there (lane 0's answer).
+__device__ __forceinline__ bool q_ready(const QueueView &q, uint32_t pos) {
+  return ld_acquire(&q.seq[pos & (q.cap - 1)]) == pos + 1;
+}
+
+// Give ticket `pos` up (lane 0): false if a donor has its slot already.
+__device__ __forceinline__ bool q_leave(const QueueView &q, uint32_t pos) {
+  return atomicCAS(&q.seq[pos & (q.cap - 1)], pos, pos + q.cap) == pos;
+}
+
+// Take the task of ticket `pos` (q_ready on lane 0 said so): put(k, word)
+// receives every word, lane-strided.
 template <typename Put>
-__device__ __forceinline__ bool q_pop(const QueueView &q, Put put) {
+__device__ __forceinline__ void q_take(const QueueView &q, uint32_t pos, Put put) {
   const uint32_t lane = lane_id();
-  uint32_t pos = 0;
-  int ok = 0;
-  if (lane == 0) {
-    pos = ld_volatile(&q.hdr->head);
-    for (int tries = 0; tries < 64; ++tries) {
-      const uint32_t s = ld_acquire(&q.seq[pos & (q.cap - 1)]);
-      const int32_t diff = (int32_t)(s - (pos + 1));
-      if (diff == 0) {
-        const uint32_t seen = atomicCAS(&q.hdr->head, pos, pos + 1);
-        if (seen == pos) {
-          ok = 1;
-          break;
-        }
-        pos = seen;
-      } else if (diff < 0) {
-        break;  // empty
-      } else {
-        pos = ld_volatile(&q.hdr->head);
-      }
-    }
-    if (ok) __threadfence();
-  }
-  ok = __shfl_sync(MCE_FULL, ok, 0);
-  if (!ok) return false;
-  pos = __shfl_sync(MCE_FULL, pos, 0);
+  __syncwarp();  // the other lanes read after lane 0's acquire
   const volatile unsigned long long *src = q.pay + (size_t)(pos & (q.cap - 1)) * q.words;
   for (uint32_t k = lane; k < q.words; k += 32) put(k, src[k]);
   __syncwarp();
   if (lane == 0) st_release(&q.seq[pos & (q.cap - 1)], pos + q.cap);  // slot free again
   __syncwarp();
-  return true;
 }
 
 // Donate a child only while more warps are waiting than tasks are queued.
 __device__ __forceinline__ bool q_wants(const QueueView &q) {
   if (!q.hdr) return false;
-  const uint32_t idle = ld_volatile(&q.hdr->idle);
-  if (idle == 0) return false;
-  const uint32_t queued = ld_volatile(&q.hdr->tail) - ld_volatile(&q.hdr->head);
-  return idle > queued;
+  return (int32_t)(ld_volatile(&q.hdr->head) - ld_volatile(&q.hdr->tail)) > 0;
 }
 
 }  // namespace mce
