@@ -58,11 +58,13 @@ struct mce_graph {
   // roots
   uint32_t *keys_in = nullptr, *keys_out = nullptr;
   int32_t *vals_in = nullptr, *roots = nullptr;
-  int32_t *hub_of = nullptr, *hub_list = nullptr;  // roots with many earlier neighbours
-  int64_t *hub_off = nullptr;                      // ... their first precomputed row
-  int32_t *hub_nx = nullptr;                       // ... and their number of distinct rows
-  unsigned long long *hub_rows = nullptr;          // ... and the rows
-  int64_t hub_off_cap = 0, hub_rows_cap = 0;
+  // rows of the roots, built before the search (EncArgs)
+  uint32_t *enc = nullptr, *enc_next = nullptr;    // enc_next: [0] whole graph, [1 + p] part p
+  unsigned long long **wptr = nullptr;
+  int32_t *nx = nullptr, *wide_list = nullptr;
+  unsigned long long *wide_off = nullptr;
+  unsigned long long *wide[1 + MAX_BATCH_PARTS] = {nullptr};  // the wide roots' rows, indexed as enc_next
+  uint64_t wide_cap[1 + MAX_BATCH_PARTS] = {0};               // ... and the words they hold
   ShapeInfo *shape = nullptr;
   void *sort_tmp = nullptr;
   size_t sort_tmp_bytes = 0;
@@ -138,13 +140,18 @@ void free_graph_bufs(mce_graph *g) {
   dfree(g->f0); dfree(g->f1); dfree(g->f2);
   dfree(g->hb0); dfree(g->hb1); dfree(g->hb2);
   dfree(g->keys_in); dfree(g->keys_out); dfree(g->vals_in); dfree(g->roots);
-  dfree(g->hub_of); dfree(g->hub_list); dfree(g->hub_off); dfree(g->hub_rows); dfree(g->hub_nx);
-  g->hub_off_cap = g->hub_rows_cap = 0;
+  dfree(g->enc); dfree(g->wptr); dfree(g->nx); dfree(g->wide_list); dfree(g->wide_off);
   dfree(g->root_nodes); dfree(g->root_count); dfree(g->root_ops);
   dfree(g->feat); dfree(g->pred); dfree(g->policy); dfree(g->wlog); dfree(g->cand);
   dfree(g->cand_n);
   g->cap_n = g->cap_m = -1;
 }
+
+// Entries for the wide roots of m arcs: each has more than 32 later (or
+// 16,384 earlier) neighbours.  Part p of a batch, from arc a on, has its own
+// from entry wide_first(a, p) on.
+inline int64_t wide_first(int64_t a, int p) { return a / 33 + p; }
+inline size_t wide_slots(int64_t m) { return (size_t)wide_first(m, MAX_PARTS) + 1; }
 
 int alloc_graph_bufs(mce_graph *g, int64_t n, int64_t m) {
   free_graph_bufs(g);
@@ -159,7 +166,8 @@ int alloc_graph_bufs(mce_graph *g, int64_t n, int64_t m) {
       (rc = dalloc(&g->hb0, N)) || (rc = dalloc(&g->hb1, N)) || (rc = dalloc(&g->hb2, N)) ||
       (rc = dalloc(&g->keys_in, N)) || (rc = dalloc(&g->keys_out, N)) ||
       (rc = dalloc(&g->vals_in, N)) || (rc = dalloc(&g->roots, N)) ||
-      (rc = dalloc(&g->hub_of, N)) || (rc = dalloc(&g->hub_list, N))) {
+      (rc = dalloc(&g->enc, M)) || (rc = dalloc(&g->wptr, N)) || (rc = dalloc(&g->nx, N)) ||
+      (rc = dalloc(&g->wide_list, wide_slots(m))) || (rc = dalloc(&g->wide_off, wide_slots(m)))) {
     free_graph_bufs(g);
     return rc;
   }
@@ -172,6 +180,7 @@ int alloc_fixed_bufs(mce_graph *g) {
   int rc;
   if ((rc = dalloc((char **)&g->peel_ctl, peel_ctl_bytes())) || (rc = dalloc(&g->shape, 1)) ||
       (rc = dalloc(&g->orient_next, 2 * (1 + MAX_PARTS))) ||
+      (rc = dalloc(&g->enc_next, 1 + MAX_PARTS)) ||
       (rc = dalloc(&g->fetch, 8)) || (rc = dalloc(&g->err, 4)) ||
       (rc = dalloc(&g->hist, MCE_HIST_MAX)) || (rc = dalloc(&g->nodes, 4)))
     return rc;
@@ -217,11 +226,6 @@ void order_graphs(int32_t *order, int64_t g0, int64_t g1, const int64_t *vo, con
     if (cx != cy) return cx < cy;
     return ao[x + 1] - ao[x] > ao[y + 1] - ao[y];
   });
-}
-
-// One search's root summary, written on the device.
-__global__ void shape_set_kernel(ShapeInfo *dst, ShapeInfo v) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *dst = v;
 }
 
 // The opt-in timeline (diagnostics only): trace_mark records an event on a
@@ -375,8 +379,8 @@ OrientArgs orient_args(mce_graph *g) {
   oa.shape = g->shape;
   oa.cost = nullptr;
   oa.sched = MCE_SCHED_PLAIN;
-  oa.hub_of = g->hub_of;
-  oa.hub_list = g->hub_list;
+  oa.wide_list = g->wide_list;
+  oa.wide_off = g->wide_off;
   oa.next = g->orient_next;
   oa.long_list = reinterpret_cast<int32_t *>(g->keys_out);  // free until the roots' sort
   return oa;
@@ -430,7 +434,7 @@ int run_parts(mce_graph *g, cudaStream_t s, int *launches, const BatchCtx *bc, i
     OrientArgs oa = orient_args(g);
     oa.v0 = vbeg;
     oa.n = vend;
-    oa.keep_shape = true;
+    oa.keep_shape = true;  // one summary, and one list of wide roots, for all parts
     oa.next = g->orient_next + 2 + 2 * p;  // the parts' orientations run at the same time
     oa.long_list = reinterpret_cast<int32_t *>(g->keys_out) + vbeg;
     if ((rc = orient_launch(oa, sp, launches))) return rc;
@@ -438,6 +442,43 @@ int run_parts(mce_graph *g, cudaStream_t s, int *launches, const BatchCtx *bc, i
   }
   for (int p = 0; p < P.k; ++p) MCE_CUDA(cudaStreamWaitEvent(s, g->part_done[p], 0));
   return MCE_OK;
+}
+
+// The rows of every root of a summary (part i - 1 of a batch, or i = 0: the
+// whole graph) before its search.  The wide roots' rows are bounded by
+// WIDE_BYTES and by what the device has left: the search encodes the rest.
+constexpr uint64_t WIDE_BYTES = 32ull << 30;
+
+int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const ShapeInfo *shape_dev,
+            int i, const int32_t *wide_list, const unsigned long long *wide_off, int64_t arc0,
+            int64_t arc1, int64_t v0, int64_t v1, cudaStream_t s, int *launches) {
+  const uint64_t want = std::min<uint64_t>(sh.wide_words, WIDE_BYTES / 8);
+  if (want > g->wide_cap[i]) {
+    dfree(g->wide[i]);
+    g->wide_cap[i] = 0;
+    for (uint64_t w = want; w > 0; w /= 2) {
+      if (cudaMalloc((void **)&g->wide[i], sizeof(unsigned long long) * w) == cudaSuccess) {
+        g->wide_cap[i] = w;
+        break;
+      }
+      g->wide[i] = nullptr;
+      (void)cudaGetLastError();  // too large for what is left: try half
+    }
+  }
+  EncArgs ea;
+  ea.n = g->n;
+  ea.rp = g->rp;
+  ea.split = g->split;
+  ea.cs = g->cs;
+  ea.roots = roots;
+  ea.shape = shape_dev;
+  ea.enc = g->enc;
+  ea.wptr = g->wptr;
+  ea.nx = g->nx;
+  ea.next = g->enc_next + i;
+  return enc_launch(ea, wide_list, sh.wide_cnt, wide_off, g->wide[i],
+                    std::min<uint64_t>(want, g->wide_cap[i]), sh.cls_cnt[CLS_R32], sh.max_dplus,
+                    arc0, arc1, v0, v1, g->sms, s, launches);
 }
 
 int read_shape(mce_graph *g, cudaStream_t s) {
@@ -624,6 +665,8 @@ int mce_graph_free(mce_graph_t g) {
   dfree(g->peel_ctl);
   dfree(g->shape);
   dfree(g->orient_next);
+  dfree(g->enc_next);
+  for (auto &w : g->wide) dfree(w);
   dfree(g->fetch);
   dfree(g->err);
   dfree(g->hist);
@@ -823,27 +866,9 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   if ((rc = read_shape(g, s))) return rc;
   const ShapeInfo &sh = g->shape_h;
   if (sh.cls_cnt[CLS_BIG]) return MCE_ELIMIT;
-  // earlier-neighbour rows of the hub roots, built by many warps at once
-  if (sh.hub_cnt > 0) {
-    const int64_t need_off = (int64_t)sh.hub_cnt + 2, need_rows = (int64_t)sh.hub_rows;
-    if (need_off > g->hub_off_cap) {
-      dfree(g->hub_off);
-      dfree(g->hub_nx);
-      g->hub_off_cap = 0;
-      if ((rc = dalloc(&g->hub_off, (size_t)need_off)) || (rc = dalloc(&g->hub_nx, (size_t)need_off)))
-        return rc;
-      g->hub_off_cap = need_off;
-    }
-    if (need_rows > g->hub_rows_cap) {
-      dfree(g->hub_rows);
-      g->hub_rows_cap = 0;
-      if ((rc = dalloc(&g->hub_rows, (size_t)need_rows))) return rc;
-      g->hub_rows_cap = need_rows;
-    }
-    if ((rc = hub_rows_launch(g->rp, g->split, g->cs, g->hub_list, sh.hub_cnt, need_rows,
-                              g->hub_off, g->hub_nx, g->hub_rows, g->sms, s, &launches)))
-      return rc;
-  }
+  if ((rc = run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0, g->n, s,
+                    &launches)))
+    return rc;
   // search scratch
   const bool share = o.worker_list != MCE_WL_OFF;
   int grid[NCLS] = {0}, block[NCLS] = {0}, smem[NCLS] = {0};
@@ -915,10 +940,9 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   a.dcap = dcap;
   a.xcap = xcap;
   a.rxcap = rxcap;
-  a.hub_of = sh.hub_cnt > 0 ? g->hub_of : nullptr;
-  a.hub_off = g->hub_off;
-  a.hub_rows = g->hub_rows;
-  a.hub_nx = g->hub_nx;
+  a.enc = g->enc;
+  a.wptr = g->wptr;
+  a.nx = g->nx;
   a.donate_min = dmin[CLS_R32];  // set per class at each launch below
   a.donate_after = (uint32_t)dafter[CLS_R32];
   a.wait_limit_ns = o.wait_limit_ms > 0 ? (uint64_t)o.wait_limit_ms * 1000000ull : IDLE_LIMIT_NS;
@@ -949,7 +973,7 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     int parts[NCLS], dmin[NCLS], dafter[NCLS];
     uint64_t wlimit;
     const void *slab, *graph_count, *graph_of, *root_nodes, *policy, *q[NCLS], *bufs[4], *wlog;
-    const void *hub[4];
+    const void *enc[3];
     int64_t n, G;
   } key;
   std::memset(&key, 0, sizeof(key));
@@ -985,10 +1009,9 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   key.bufs[1] = g->split;
   key.bufs[2] = g->cs;
   key.bufs[3] = g->roots;
-  key.hub[0] = a.hub_of;
-  key.hub[1] = a.hub_off;
-  key.hub[2] = a.hub_rows;
-  key.hub[3] = a.hub_nx;
+  key.enc[0] = a.enc;
+  key.enc[1] = a.wptr;
+  key.enc[2] = a.nx;
   key.n = g->n;
   key.G = bc ? bc->G : 0;
   static_assert(sizeof(SearchKey) <= sizeof(g->search_key), "search key");
@@ -1140,7 +1163,7 @@ namespace {
 // mce_batch_count_host, pipelined: each part of a batch arriving from the
 // host is rebased, peeled, oriented and its roots sorted on a stream of its
 // own as soon as its copy lands; the host reads the part's summary and
-// queues its search (hub rows, then the engine classes) on the call's stream,
+// queues its rows (enc.cu) and its search on the call's stream,
 // so part p is searched while parts p+1.. are still being copied and peeled.
 // A part's graphs share no vertex with other parts, so its search reads only
 // its own rows.  Buffers that a later part outgrows are replaced and the old
@@ -1154,12 +1177,11 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
   int launches = 0, rc = MCE_OK;
   mce_stats_t st;
   std::memset(&st, 0, sizeof(st));
-  // part shapes: [0, MAX_PARTS) the parts', [MAX_PARTS, 2 MAX_PARTS) their searches',
-  // [2 MAX_PARTS] the deferred roots'
-  if (!g->part_shape && (rc = dalloc(&g->part_shape, 2 * MAX_PARTS + 1))) return rc;
+  // part shapes: [0, MAX_PARTS) the parts', [MAX_PARTS] the deferred roots'
+  if (!g->part_shape && (rc = dalloc(&g->part_shape, MAX_PARTS + 1))) return rc;
   if (!g->part_fetch && (rc = dalloc(&g->part_fetch, 8 * (MAX_PARTS + 1)))) return rc;
   if (!g->part_shape_h &&
-      cudaHostAlloc((void **)&g->part_shape_h, sizeof(ShapeInfo) * (2 * MAX_PARTS + 1),
+      cudaHostAlloc((void **)&g->part_shape_h, sizeof(ShapeInfo) * (MAX_PARTS + 1),
                     cudaHostAllocDefault) != cudaSuccess)
     return MCE_ENOMEM;
   for (int p = 0; p < P.k; ++p) {
@@ -1223,20 +1245,19 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     oa.v0 = vbeg;
     oa.n = vend;
     oa.shape = g->part_shape + p;
-    oa.hub_list = g->hub_list + vbeg;  // hub indices are the part's own
+    oa.wide_list = g->wide_list + wide_first(P.ao_h[P.g[p]], p);
+    oa.wide_off = g->wide_off + wide_first(P.ao_h[P.g[p]], p);
     oa.next = g->orient_next + 2 + 2 * p;
     oa.long_list = reinterpret_cast<int32_t *>(g->keys_out) + vbeg;
     if ((rc = orient_launch(oa, sp, &launches))) return rc;
     const int64_t np = vend - vbeg;
-    // keys: class, hubs first, then (degree order) the cost; vertex order
-    // within a key (plain order: no cost)
-    if (np > 0 && (rc = rekey_launch(np, g->keys_in + vbeg, nullptr, g->rp + vbeg,
-                                     g->split + vbeg, nullptr, degree ? heavy : 1e30f,
-                                     degree ? heavy : 1e30f, g->sms, sp, &launches, 0,
-                                     g->hub_of + vbeg)))
+    // keys: class, then (degree order) the cost; vertex order within a key
+    if (np > 0 && degree &&
+        (rc = rekey_launch(np, g->keys_in + vbeg, nullptr, g->rp + vbeg, g->split + vbeg, nullptr,
+                           heavy, heavy, g->sms, sp, &launches)))
       return rc;
     if ((rc = roots_sort(np, g->keys_in + vbeg, g->keys_out + vbeg, g->vals_in + vbeg,
-                         g->roots + vbeg, 32, &g->part_tmp[p], &g->part_tmp_bytes[p],
+                         g->roots + vbeg, degree ? 32 : 3, &g->part_tmp[p], &g->part_tmp_bytes[p],
                          g->part_shape + p, sp, &launches)))
       return rc;
     MCE_CUDA(cudaMemcpyAsync(g->part_shape_h + p, g->part_shape + p, sizeof(ShapeInfo),
@@ -1245,23 +1266,19 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     trace_mark(g, sp, "prep", p);
     return MCE_OK;
   };
-  // The searches, in order on the call's stream.  As each part lands, its
-  // 32-bit roots without hub rows are searched (most of the work).  Every
-  // other root - the hubs of all classes, the 64-bit and wide classes, whose
-  // largest trees set a launch's tail - waits for one search at the end,
-  // with one hub table built over all parts: one tail instead of one per part.
+  // The searches, in order on the call's stream.  As each part lands, the rows
+  // of its roots are built and its 32-bit roots are searched (most of the
+  // work).  The 64-bit and wide classes, whose largest trees set a launch's
+  // tail, wait for one search at the end: one tail instead of one per part.
   uint32_t err_limit = 0;
   const bool share_q = share;
   const int wbits = o.bitmap_width == 64 ? 64 : 32;
-  ShapeInfo *sh_search = g->part_shape + MAX_PARTS;   // [MAX_PARTS]: per-part searches
-  ShapeInfo *sh_final = g->part_shape + 2 * MAX_PARTS;
-  ShapeInfo *hs_final = g->part_shape_h + 2 * MAX_PARTS;
+  ShapeInfo *sh_final = g->part_shape + MAX_PARTS;
+  ShapeInfo *hs_final = g->part_shape_h + MAX_PARTS;
   struct Seg {
     int64_t at, cnt;
   };
-  std::vector<Seg> defer[3];  // by class: R32 hubs, R64, MEM (offsets into g->roots)
-  std::vector<Seg> hubsegs;   // the parts' hub lists (offsets into g->hub_list)
-  uint64_t hub_rows_total = 0;
+  std::vector<Seg> defer[2];  // by class: R64, MEM (offsets into g->roots)
   uint32_t mx_dplus = 0, mx_dm_mem = 0, mx_dm_reg = 0, mx_deg = 0;
   // grid, slab and queue of one class launch; returns MCE_OK or an error
   auto plan = [&](int c, int64_t roots, int dcap, int xcap, int rxcap, int *grid, int *block,
@@ -1319,6 +1336,9 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     a.prio = g->prio;
     a.x_pivot = (o.x_pivot || o.induced == MCE_INDUCED_PX) ? 1 : 0;
     a.stage = o.stage_lists ? 1 : 0;
+    a.enc = g->enc;
+    a.wptr = g->wptr;
+    a.nx = g->nx;
   };
   auto run_class = [&](int c, BKArgs &a, int grid, int block, int smem, int parts_c, int dmin_c,
                        int dafter_c, const QueueView &qv, int dcap, int xcap, int rxcap) -> int {
@@ -1343,13 +1363,10 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       return MCE_OK;
     }
     const int64_t vbeg = vb[p];
-    // roots of the part, class-sorted, hubs first within a class
-    const int64_t n32 = (int64_t)sh.cls_cnt[CLS_R32] - sh.hub_r32;
-    defer[0].push_back({vbeg + sh.cls_off[CLS_R32], (int64_t)sh.hub_r32});
-    defer[1].push_back({vbeg + sh.cls_off[CLS_R64], (int64_t)sh.cls_cnt[CLS_R64]});
-    defer[2].push_back({vbeg + sh.cls_off[CLS_MEM], (int64_t)sh.cls_cnt[CLS_MEM]});
-    hubsegs.push_back({vbeg, (int64_t)sh.hub_cnt});
-    hub_rows_total += sh.hub_rows;
+    // roots of the part, class-sorted
+    const int64_t n32 = (int64_t)sh.cls_cnt[CLS_R32];
+    defer[0].push_back({vbeg + sh.cls_off[CLS_R64], (int64_t)sh.cls_cnt[CLS_R64]});
+    defer[1].push_back({vbeg + sh.cls_off[CLS_MEM], (int64_t)sh.cls_cnt[CLS_MEM]});
     mx_dplus = std::max(mx_dplus, sh.max_dplus);
     mx_dm_mem = std::max(mx_dm_mem, sh.max_dminus_mem);
     mx_dm_reg = std::max(mx_dm_reg, sh.max_dminus_reg);
@@ -1358,26 +1375,24 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     for (int c = 0; c < NCLS && c < 8; ++c) st.class_roots[c] += sh.cls_cnt[c];
     if ((int32_t)sh.max_dplus > st.max_later_degree) st.max_later_degree = (int32_t)sh.max_dplus;
     if ((int64_t)sh.max_deg > st.max_degree) st.max_degree = sh.max_deg;
+    const int64_t arc0 = P.ao_h[P.g[p]], arc1 = P.ao_h[P.g[p + 1]];
+    const int64_t wf = wide_first(arc0, p);
+    if ((rc = run_enc(g, sh, g->roots + vbeg, g->part_shape + p, 1 + p, g->wide_list + wf,
+                      g->wide_off + wf, arc0, arc1, vbeg, vb[p + 1], s, &launches)))
+      return rc;
+    trace_mark(g, s, "rows", p);
     if (n32 <= 0) return MCE_OK;
-    // the part's 32-bit roots after its hubs: earlier degree <= HUB_XMIN, no hub rows
-    ShapeInfo ss{};
-    for (int c = 1; c < 9; ++c) ss.cls_off[c] = (uint32_t)n32;
-    ss.cls_cnt[CLS_R32] = (uint32_t)n32;
-    // written by a kernel rather than copied from the host on the call's
-    // stream, whose copy would share the copy engine with the part copies
-    // still in flight (0.3 ms end to end)
-    shape_set_kernel<<<1, 32, 0, s>>>(sh_search + p, ss);
-    MCE_CUDA(cudaGetLastError());
-    launches += 1;
-    const int dcap = 32, xcap = 1, rxcap = REG_XCAP;
+    const int dcap = 32, xcap = 1;
+    int rxcap = REG_XCAP;
+    while (rxcap < (int)sh.max_dminus_reg && rxcap < REG_XCAP_MAX) rxcap <<= 1;
     int grid = 0, block = 0, smem = 0, pc = 1, dm = 0, da = 0;
     QueueView qv;
     if ((rc = plan(CLS_R32, n32, dcap, xcap, rxcap, &grid, &block, &smem, &pc, &dm, &da, &qv)))
       return rc;
     BKArgs a;
     base_args(a, dcap, xcap, rxcap);
-    a.roots = g->roots + vbeg + sh.cls_off[CLS_R32] + sh.hub_r32;
-    a.shape = sh_search + p;
+    a.roots = g->roots + vbeg;
+    a.shape = g->part_shape + p;
     a.fetch = g->part_fetch + 8 * p;
     trace_mark(g, s, "sb", p);
     if ((rc = run_class(CLS_R32, a, grid, block, smem, pc, dm, da, qv, dcap, xcap, rxcap)))
@@ -1414,14 +1429,13 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     std::this_thread::yield();
   }
   if (bad) return finish(MCE_ECUDA);
-  // the deferred roots of every part: one list (R32 hubs, R64, MEM) in the
-  // sort's key buffer and one hub list in its value buffer, both free now
-  int64_t ncls[3] = {0, 0, 0};
+  // the deferred roots of every part: one list (R64, MEM) in the sort's key
+  // buffer, free now
+  int64_t ncls[2] = {0, 0};
   int32_t *dlist = reinterpret_cast<int32_t *>(g->keys_out);
-  int32_t *hlist = g->vals_in;
   if (!err_limit) {
     int64_t at = 0;
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 2; ++c)
       for (const Seg &sg : defer[c]) {
         if (sg.cnt > 0)
           MCE_CUDA(cudaMemcpyAsync(dlist + at, g->roots + sg.at, sizeof(int32_t) * (size_t)sg.cnt,
@@ -1430,57 +1444,12 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
         ncls[c] += sg.cnt;
       }
     trace_mark(g, s, "defer");
-    int64_t nh = 0;
-    for (const Seg &sg : hubsegs) {
-      if (sg.cnt > 0)
-        MCE_CUDA(cudaMemcpyAsync(hlist + nh, g->hub_list + sg.at, sizeof(int32_t) * (size_t)sg.cnt,
-                                 cudaMemcpyDeviceToDevice, s));
-      nh += sg.cnt;
-    }
-    if (nh > 0) {
-      if ((rc = hub_index_launch(hlist, (uint32_t)nh, g->hub_of, s, &launches))) return finish(rc);
-      const int64_t need_off = nh + 2, need_rows = (int64_t)hub_rows_total;
-      if (need_off > g->hub_off_cap) {
-        if (g->hub_off) retired.push_back(g->hub_off);
-        if (g->hub_nx) retired.push_back(g->hub_nx);
-        g->hub_off = nullptr;
-        g->hub_nx = nullptr;
-        g->hub_off_cap = 0;
-        if ((rc = dalloc(&g->hub_off, (size_t)need_off)) ||
-            (rc = dalloc(&g->hub_nx, (size_t)need_off)))
-          return finish(rc);
-        g->hub_off_cap = need_off;
-      }
-      if (need_rows > g->hub_rows_cap) {
-        if (g->hub_rows) retired.push_back(g->hub_rows);
-        g->hub_rows = nullptr;
-        g->hub_rows_cap = 0;
-        if ((rc = dalloc(&g->hub_rows, (size_t)need_rows))) return finish(rc);
-        g->hub_rows_cap = need_rows;
-      }
-      if ((rc = hub_rows_launch(g->rp, g->split, g->cs, hlist, (uint32_t)nh, need_rows,
-                                g->hub_off, g->hub_nx, g->hub_rows, g->sms, s, &launches)))
-        return finish(rc);
-    }
-    trace_mark(g, s, "hubrows");
-    const int64_t nd = ncls[0] + ncls[1] + ncls[2];
+    const int64_t nd = ncls[0] + ncls[1];
     if (nd > 0) {
-      // the 32-bit hubs run in the 64-bit launch, ahead of its roots: one
-      // launch and one tail less (48.1 against 49.3 ms end to end on the
-      // 4,096-graph batch; the 64-bit engine takes any root of d+ <= 64)
-      const bool fold = ncls[0] > 0 && ncls[1] > 0;
-      int64_t nrun[3] = {ncls[0], ncls[1], ncls[2]};
-      if (fold) {
-        nrun[1] += nrun[0];
-        nrun[0] = 0;
-      }
       ShapeInfo fs{};
-      fs.cls_cnt[CLS_R32] = (uint32_t)nrun[0];
-      fs.cls_cnt[CLS_R64] = (uint32_t)nrun[1];
-      fs.cls_cnt[CLS_MEM] = (uint32_t)nrun[2];
-      fs.cls_off[CLS_R32] = 0;
-      fs.cls_off[CLS_R64] = (uint32_t)nrun[0];
-      fs.cls_off[CLS_MEM] = (uint32_t)(ncls[0] + ncls[1]);
+      fs.cls_cnt[CLS_R64] = (uint32_t)ncls[0];
+      fs.cls_cnt[CLS_MEM] = (uint32_t)ncls[1];
+      fs.cls_off[CLS_MEM] = (uint32_t)ncls[0];
       for (int c = CLS_MEM + 1; c < 9; ++c) fs.cls_off[c] = (uint32_t)nd;
       hs_final[0] = fs;
       MCE_CUDA(cudaMemcpyAsync(sh_final, hs_final, sizeof(ShapeInfo), cudaMemcpyHostToDevice, s));
@@ -1488,12 +1457,11 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       const int xcap = (int)(mx_dm_mem > 0 ? mx_dm_mem : 1);
       int rxcap = REG_XCAP;
       while (rxcap < (int)mx_dm_reg && rxcap < REG_XCAP_MAX) rxcap <<= 1;
-      const int cls_of[3] = {CLS_R32, CLS_R64, CLS_MEM};
-      int grid[3] = {0}, block[3] = {0}, smem[3] = {0}, pc[3] = {1, 1, 1}, dm[3] = {0},
-          da[3] = {0};
-      QueueView qv[3];
-      for (int i = 0; i < 3; ++i)
-        if (nrun[i] > 0 && (rc = plan(cls_of[i], nrun[i], dcap, xcap, rxcap, &grid[i], &block[i],
+      const int cls_of[2] = {CLS_R64, CLS_MEM};
+      int grid[2] = {0}, block[2] = {0}, smem[2] = {0}, pc[2] = {1, 1}, dm[2] = {0}, da[2] = {0};
+      QueueView qv[2];
+      for (int i = 0; i < 2; ++i)
+        if (ncls[i] > 0 && (rc = plan(cls_of[i], ncls[i], dcap, xcap, rxcap, &grid[i], &block[i],
                                       &smem[i], &pc[i], &dm[i], &da[i], &qv[i])))
           return finish(rc);
       BKArgs a;
@@ -1501,12 +1469,8 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       a.roots = dlist;
       a.shape = sh_final;
       a.fetch = g->part_fetch + 8 * MAX_PARTS;
-      a.hub_of = nh > 0 ? g->hub_of : nullptr;
-      a.hub_off = g->hub_off;
-      a.hub_rows = g->hub_rows;
-      a.hub_nx = g->hub_nx;
-      for (int i : {2, 1, 0})  // wide, 64-bit, then the 32-bit hubs
-        if (nrun[i] > 0 && (rc = run_class(cls_of[i], a, grid[i], block[i], smem[i], pc[i], dm[i],
+      for (int i : {1, 0})  // wide, then 64-bit
+        if (ncls[i] > 0 && (rc = run_class(cls_of[i], a, grid[i], block[i], smem[i], pc[i], dm[i],
                                            da[i], qv[i], dcap, xcap, rxcap)))
           return finish(rc);
     }

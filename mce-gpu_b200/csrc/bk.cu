@@ -297,225 +297,7 @@ __global__ void __launch_bounds__(MEM_BLOCK, MINB) bk_mem_kernel(BKArgs a, int c
   }
 }
 
-// ---------------------------------------------------------------------------
-// Hub rows: the earlier-neighbour rows of roots with d- > HUB_XMIN, built
-// before the search by many warps at once (the root's own warp would walk
-// thousands of later lists one window at a time, a chain of dependent
-// loads that leaves the rest of its class idle at the end).
-// ---------------------------------------------------------------------------
-constexpr int HUB_BLOCK = 256;
-constexpr int HUB_FETCH = 4;  // 32-row chunks a warp of hub_rows_kernel takes at a time
-
-// off[j] = sum over k < j of hub k's earlier degree rounded up to 32; one
-// block of HUB_OFF_BLOCK threads walks the list in tiles of HUB_OFF_PER
-// hubs per thread (their offsets gathered together), scanning each tile.
-constexpr int HUB_OFF_BLOCK = 1024, HUB_OFF_PER = 8;
-__global__ void __launch_bounds__(HUB_OFF_BLOCK) hub_offsets_kernel(
-    const int32_t *__restrict__ rp, const int32_t *__restrict__ split,
-    const int32_t *__restrict__ hub_list, uint32_t cnt, int64_t *__restrict__ off,
-    int32_t *__restrict__ nx) {
-  __shared__ long long wsum[HUB_OFF_BLOCK / 32];
-  __shared__ long long carry;
-  const int lane = (int)lane_id(), wid = (int)(threadIdx.x >> 5);
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < cnt; base += HUB_OFF_BLOCK * HUB_OFF_PER) {
-    const uint32_t j0 = base + threadIdx.x * HUB_OFF_PER;
-    long long v[HUB_OFF_PER];
-    long long mine = 0;
-#pragma unroll
-    for (int k = 0; k < HUB_OFF_PER; ++k) {
-      v[k] = 0;
-      if (j0 + k < cnt) {
-        const int32_t r = hub_list[j0 + k];
-        v[k] = (long long)(((uint32_t)(split[r] - rp[r]) + 31u) & ~31u);
-      }
-      mine += v[k];
-    }
-    long long x = mine;  // inclusive scan of the threads' sums in the warp
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long y = __shfl_up_sync(MCE_FULL, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[wid] = x;
-    __syncthreads();
-    long long before = carry + x - mine;
-    for (int w = 0; w < wid; ++w) before += wsum[w];
-#pragma unroll
-    for (int k = 0; k < HUB_OFF_PER; ++k) {
-      if (j0 + k < cnt) {
-        off[j0 + k] = (int64_t)before;
-        nx[j0 + k] = -1;
-      }
-      before += v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == HUB_OFF_BLOCK - 1) carry = before;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    off[cnt] = (int64_t)carry;
-    off[cnt + 1] = 0;  // hub_rows_kernel's chunk counter
-  }
-}
-
-struct HubSmem {
-  int32_t hkey[256];  // hash of the hub's later list (<= 64 ids): vertex id (-1: empty) ...
-  uint8_t hidx[256];  // ... and its index in the list
-  u64 xs[32];         // the rows of the current 32 earlier neighbours
-  int32_t off[32], beg[32], own[64];  // flattened-walk scratch (two windows)
-};
-
-// flat_walk (engine.cuh) two windows at a time: the two elements of a lane
-// are loaded together, so a warp keeps two reads of the lists in flight.
-template <typename F>
-__device__ __forceinline__ void flat_walk2(const int32_t *__restrict__ cs, int32_t b, int len,
-                                           int32_t *off_sm, int32_t *beg_sm, int32_t *own_sm,
-                                           F f) {
-  const int lane = (int)lane_id();
-  const int incl = warp_incl_scan(len);
-  const int T = __shfl_sync(MCE_FULL, incl, 31);
-  const int off = incl - len;
-  off_sm[lane] = off;
-  beg_sm[lane] = b;
-  int carry = 0;
-  for (int e0 = 0; e0 < T; e0 += 64) {
-    const bool stA = len > 0 && off >= e0 && off < e0 + 32;
-    const bool stB = len > 0 && off >= e0 + 32 && off < e0 + 64;
-    if (stA) own_sm[off - e0] = lane;
-    if (stB) own_sm[off - e0] = lane;  // 32 .. 63: window B
-    const uint32_t mA = __reduce_or_sync(MCE_FULL, stA ? 1u << (off - e0) : 0u);
-    const uint32_t mB = __reduce_or_sync(MCE_FULL, stB ? 1u << (off - e0 - 32) : 0u);
-    __syncwarp();
-    const uint32_t keep = 0xFFFFFFFFu >> (31 - lane);
-    const uint32_t bA = mA & keep, bB = mB & keep;
-    const int tA = bA ? own_sm[31 - __clz(bA)] : carry;
-    const int cA = __shfl_sync(MCE_FULL, tA, 31);
-    const int tB = bB ? own_sm[32 + 31 - __clz(bB)] : cA;
-    carry = __shfl_sync(MCE_FULL, tB, 31);
-    const int eA = e0 + lane, eB = e0 + 32 + lane;
-    int32_t wA = -1, wB = -1;
-    if (eA < T) wA = cs[beg_sm[tA] + (eA - off_sm[tA])];
-    if (eB < T) wB = cs[beg_sm[tB] + (eB - off_sm[tB])];
-    if (eA < T) f(tA, wA);
-    if (eB < T) f(tB, wB);
-    __syncwarp();
-  }
-}
-
-__device__ __forceinline__ uint32_t hub_slot(int32_t w) { return ((uint32_t)w * 0x9E3779B1u) >> 24; }
-
-// Warps fetch HUB_FETCH 32-row chunks at a time from a counter (off[cnt + 1],
-// zeroed by hub_offsets_kernel), so a warp whose chunks walk long lists takes
-// fewer; the hash of a hub's later list (d+ <= 64) is rebuilt when a warp's
-// chunks move on to the next hub (a warp's chunks only move forward).
-__global__ void __launch_bounds__(HUB_BLOCK) hub_rows_kernel(
-    const int32_t *__restrict__ rp, const int32_t *__restrict__ split,
-    const int32_t *__restrict__ cs, const int32_t *__restrict__ hub_list, uint32_t cnt,
-    const int64_t *__restrict__ off, int64_t chunks, unsigned long long *__restrict__ rows,
-    unsigned long long *next) {
-  __shared__ HubSmem sm_all[HUB_BLOCK / 32];
-  HubSmem &sm = sm_all[threadIdx.x >> 5];
-  const int lane = (int)lane_id();
-  int32_t cur = -1;  // hub whose hash is built
-  uint32_t j = 0;
-  int64_t c = 0, c1 = 0;
-  for (;;) {
-    if (c == c1) {
-      unsigned long long f = 0;
-      if (lane == 0) f = atomicAdd(next, (unsigned long long)HUB_FETCH);
-      c = (int64_t)__shfl_sync(MCE_FULL, f, 0);
-      if (c >= chunks) break;
-      c1 = min(chunks, c + HUB_FETCH);
-    }
-    const int64_t row0 = 32 * c++;
-    if (cur < 0 || row0 >= off[j + 1]) {  // first chunk, or the next hub: last j with off[j] <= row0
-      uint32_t lo = 0, hi = cnt - 1;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= row0) lo = mid; else hi = mid - 1;
-      }
-      j = lo;
-      cur = hub_list[j];
-      const int32_t sb = split[cur], d = rp[cur + 1] - sb;
-      for (int i = lane; i < 256; i += 32) sm.hkey[i] = -1;
-      __syncwarp();
-      for (int i = lane; i < d; i += 32) {  // the later list's ids are distinct
-        const int32_t w = cs[sb + i];
-        uint32_t h = hub_slot(w);
-        while (atomicCAS(&sm.hkey[h], -1, w) != -1) h = (h + 1) & 255u;
-        sm.hidx[h] = (uint8_t)i;
-      }
-      __syncwarp();
-    }
-    const int32_t ub = rp[cur], u = split[cur] - ub;
-    const int64_t i0 = row0 - off[j];
-    const int items = (int)min((int64_t)32, (int64_t)u - i0);
-    int xb = 0, xlen = 0;
-    if (lane < items) {
-      const int32_t x = cs[ub + i0 + lane];
-      xb = split[x];
-      xlen = rp[x + 1] - xb;
-    }
-    sm.xs[lane] = 0;
-    __syncwarp();
-    flat_walk2(cs, xb, xlen, sm.off, sm.beg, sm.own, [&](int t, int32_t w) {
-      uint32_t h = hub_slot(w);
-      for (;;) {
-        const int32_t k = sm.hkey[h];
-        if (k == w) {
-          atomicOr(&sm.xs[t], 1ull << sm.hidx[h]);
-          break;
-        }
-        if (k == -1) break;
-        h = (h + 1) & 255u;
-      }
-    });
-    __syncwarp();
-    rows[row0 + lane] = sm.xs[lane];  // lanes past the hub's list write its zero padding
-    __syncwarp();
-  }
-}
-
 }  // namespace
-
-
-namespace {
-__global__ void hub_index_kernel(const int32_t *__restrict__ list, uint32_t cnt, int32_t *hub_of) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x)
-    hub_of[list[i]] = (int32_t)i;
-}
-}  // namespace
-
-int hub_index_launch(const int32_t *list, uint32_t cnt, int32_t *hub_of, cudaStream_t s,
-                     int *launches) {
-  if (cnt == 0) return MCE_OK;
-  hub_index_kernel<<<(cnt + 255) / 256 < 1184 ? (cnt + 255) / 256 : 1184, 256, 0, s>>>(list, cnt,
-                                                                                   hub_of);
-  MCE_CUDA(cudaGetLastError());
-  if (launches) *launches += 1;
-  return MCE_OK;
-}
-
-int hub_rows_launch(const int32_t *rp, const int32_t *split, const int32_t *cs,
-                    const int32_t *hub_list, uint32_t cnt, int64_t total_rows, int64_t *off,
-                    int32_t *nx, unsigned long long *rows, int sms, cudaStream_t s,
-                    int *launches) {
-  if (cnt == 0) return MCE_OK;
-  hub_offsets_kernel<<<1, HUB_OFF_BLOCK, 0, s>>>(rp, split, hub_list, cnt, off, nx);
-  MCE_CUDA(cudaGetLastError());
-  const int64_t chunks = total_rows / 32;
-  int64_t blocks = ((chunks + 7) / 8 + 0);  // up to one chunk per warp
-  const int64_t cap = (int64_t)sms * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  hub_rows_kernel<<<(unsigned)blocks, HUB_BLOCK, 0, s>>>(
-      rp, split, cs, hub_list, cnt, off, chunks, rows,
-      reinterpret_cast<unsigned long long *>(off + cnt + 1));
-  MCE_CUDA(cudaGetLastError());
-  if (launches) *launches += 2;
-  return MCE_OK;
-}
 
 size_t bk_slab_words(int cls, int dcap, int xcap, int rxcap) {
   if (cls == CLS_R32 || cls == CLS_R64) return 4 * (size_t)rxcap;  // hash, rows, leaf list

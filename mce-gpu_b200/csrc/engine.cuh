@@ -364,6 +364,94 @@ struct RegRoot {
   Word r0 = 0, r1 = 0;
 };
 
+// A root whose rows were built before the search: at its CSR positions
+// (enc, 32-bit words) or in its region (wrows).  The distinct non-empty
+// earlier rows go to sl.xr in list order; more than 32 of them are
+// deduplicated once: the first warp to load the root writes the distinct ones
+// back over the built ones and publishes their number (nx), so the warps that
+// take its subtrees later only copy them.
+template <typename Word, int NR>
+__device__ __forceinline__ void reg_load(const BKArgs &a, RegSmem<Word, NR> &sm,
+                                         const RegSlab<Word> &sl, int32_t r, int32_t ub, int u,
+                                         int32_t sb, int d, uint32_t *enc,
+                                         unsigned long long *wrows, RegRoot<Word> &rt) {
+  const int lane = (int)lane_id();
+  const uint32_t lt = (1u << lane) - 1u;
+  auto earlier = [&](int i) -> Word {  // from L2: another warp may have rewritten them
+    return enc ? (Word)__ldcg(enc + ub + i) : (Word)__ldcg(wrows + d + i);
+  };
+  rt.r = r;
+  rt.d = d;
+  rt.r0 = lane < d ? (enc ? (Word)enc[sb + lane] : (Word)wrows[lane]) : (Word)0;
+  rt.r1 = 0;
+  if constexpr (NR == 2) {
+    if (lane + 32 < d) rt.r1 = (Word)wrows[lane + 32];
+  }
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    const int i = lane + 32 * k;
+    sm.pl[i] = i < d ? a.cs[sb + i] : INT_MAX;
+  }
+  if (u <= 32) {
+    const Word row = lane < u ? earlier(lane) : (Word)0;
+    const uint32_t same = __match_any_sync(MCE_FULL, row);
+    const bool fresh = row != 0 && (same & lt) == 0;  // first lane of its value
+    const uint32_t mk = __ballot_sync(MCE_FULL, fresh);
+    if (fresh) sl.xr[__popc(mk & lt)] = row;
+    rt.nX = __popc(mk);
+    __syncwarp();
+    return;
+  }
+  int kept = -1;
+  if (lane == 0) kept = (int)ld_acquire(reinterpret_cast<const uint32_t *>(a.nx + r));
+  kept = __shfl_sync(MCE_FULL, kept, 0);
+  __syncwarp();  // the other lanes read after lane 0's acquire
+  if (kept >= 0) {
+    for (int i = lane; i < kept; i += 32) sl.xr[i] = earlier(i);
+    rt.nX = kept;
+    __syncwarp();
+    return;
+  }
+  int hc = 32, nX = 0;
+  while (hc < 2 * u && hc < 2 * sl.xc) hc <<= 1;
+  for (int i = lane; i < hc; i += 32) sl.hash[i] = 0;
+  __syncwarp();
+  for (int i0 = 0; i0 < u; i0 += 32) {
+    const Word row = i0 + lane < u ? earlier(i0 + lane) : (Word)0;
+    bool fresh = false;
+    if (row != 0) {
+      uint32_t h = hash_word((u64)row) & (uint32_t)(hc - 1);
+      for (int probe = 0; probe < hc; ++probe) {
+        const Word old = atomicCAS(&sl.hash[h], (Word)0, row);
+        if (old == 0) {
+          fresh = true;
+          break;
+        }
+        if (old == row) break;
+        h = (h + 1) & (uint32_t)(hc - 1);
+      }
+    }
+    const uint32_t mk = __ballot_sync(MCE_FULL, fresh);
+    if (fresh) sl.xr[nX + __popc(mk & lt)] = row;
+    nX += __popc(mk);
+    __syncwarp();
+  }
+  rt.nX = nX;
+  // with several warps per root two of them may load it at once, so then the
+  // rows stay as built and every warp deduplicates them itself
+  if (a.parts <= 1) {
+    for (int i = lane; i < nX; i += 32) {
+      if (enc)
+        enc[ub + i] = (uint32_t)sl.xr[i];
+      else
+        wrows[d + i] = (u64)sl.xr[i];
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) st_release(reinterpret_cast<uint32_t *>(a.nx + r), (uint32_t)nX);
+  }
+}
+
 // STAGE: the lists are staged in shared memory by bulk copies (*stg).
 template <typename Word, int NR, bool STAGE = false>
 __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<Word> &sl,
@@ -382,6 +470,21 @@ __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab
     rt.r = r;
     rt.d = 0;
     rt.nX = 0;
+    return;
+  }
+  // Rows built before the search (enc.cu): adjacency rows and earlier rows are
+  // read, not walked for.  A root past the regions' limit has none; with
+  // staged lists only the roots with many earlier neighbours read theirs.
+  uint32_t *enc = nullptr;
+  unsigned long long *wrows = nullptr;
+  if (a.enc && (!STAGE || u > 256)) {
+    if (d <= 32)
+      enc = a.enc;
+    else
+      wrows = a.wptr[r];
+  }
+  if (enc || wrows) {
+    reg_load<Word, NR>(a, sm, sl, r, ub, u, sb, d, enc, wrows, rt);
     return;
   }
 
@@ -465,22 +568,7 @@ __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab
   // in N+(x).  Up to 32 of them are deduplicated with one match over the
   // warp; more go through a hash set in the slab.
   int nX = 0;
-  // A hub's rows were built before the search (hub_rows_launch); its first
-  // encode writes the distinct ones back there and publishes their number
-  // (hub_nx), so the warps that take its subtrees later only copy them.
-  const int32_t hub = (u > 0 && a.hub_of) ? a.hub_of[r] : -1;
-  unsigned long long *hrows = hub >= 0 ? a.hub_rows + a.hub_off[hub] : nullptr;
-  int kept = -1;
-  if (hrows) {
-    if (lane == 0) kept = (int)ld_acquire(reinterpret_cast<const uint32_t *>(a.hub_nx + hub));
-    kept = __shfl_sync(MCE_FULL, kept, 0);
-    __syncwarp();  // the other lanes read after lane 0's acquire
-  }
-  if (kept >= 0) {
-    for (int i = lane; i < kept; i += 32) sl.xr[i] = (Word)__ldcg(hrows + i);  // from L2
-    __syncwarp();
-    nX = kept;
-  } else if (u > 0) {
+  if (u > 0) {
     const bool hashed = u > 32;
     int hc = 32;
     if (hashed) {
@@ -489,25 +577,20 @@ __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab
     }
     for (int c = 0; c * 32 < u; ++c) {
       const int items = min(32, u - c * 32);
-      Word row;
-      if (hrows) {
-        row = (Word)hrows[c * 32 + lane];  // zero past the list (padding)
-      } else {
-        int xb = 0, xlen = 0;
-        if (lane < items) {
-          const int32_t x = a.cs[ub + c * 32 + lane];
-          xb = a.split[x];
-          xlen = a.rp[x + 1] - xb;
-        }
-        sm.xs[lane] = 0;
-        __syncwarp();
-        walk(xb, xlen, [&](int t, int32_t w) {
-          const int i = p_find(sm, w);
-          if (i >= 0) atomicOr(&sm.xs[t], O::bit(i));
-        });
-        __syncwarp();
-        row = sm.xs[lane];
+      int xb = 0, xlen = 0;
+      if (lane < items) {
+        const int32_t x = a.cs[ub + c * 32 + lane];
+        xb = a.split[x];
+        xlen = a.rp[x + 1] - xb;
       }
+      sm.xs[lane] = 0;
+      __syncwarp();
+      walk(xb, xlen, [&](int t, int32_t w) {
+        const int i = p_find(sm, w);
+        if (i >= 0) atomicOr(&sm.xs[t], O::bit(i));
+      });
+      __syncwarp();
+      const Word row = sm.xs[lane];
       bool fresh = false;
       if (!hashed) {
         const uint32_t same = __match_any_sync(MCE_FULL, row);
@@ -528,15 +611,6 @@ __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab
       if (fresh) sl.xr[nX + __popc(mk & lt)] = row;
       nX += __popc(mk);
       __syncwarp();
-    }
-    // rows [0, nX) of the hub's region are no longer read as built; with
-    // several warps per root two of them may encode the hub at once, so
-    // then the rows stay as built and every warp deduplicates them itself
-    if (hrows && a.parts <= 1) {
-      for (int i = lane; i < nX; i += 32) hrows[i] = (u64)sl.xr[i];
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) st_release(reinterpret_cast<uint32_t *>(a.hub_nx + hub), (uint32_t)nX);
     }
   }
   rt.r = r;
@@ -1239,7 +1313,8 @@ __device__ __forceinline__ int wide_find(const Slab &sl, int pc, int32_t w) {
 struct MemRoot {
   int32_t r = -1;
   int d = 0, Wr = 0, nX = 0;
-  const u64 *rows = nullptr;  // the induced rows: shared memory when d+ <= MEM_SROWS_D, else the slab
+  const u64 *rows = nullptr;  // the induced rows: shared memory when d+ <= MEM_SROWS_D, else global
+  const u64 *xr = nullptr;    // the earlier neighbours' rows
 };
 
 // Roots of the wide engine with at most this many later neighbours keep their
@@ -1263,9 +1338,22 @@ __device__ void mem_encode(const BKArgs &a, MemSmem &sm, const Slab &sl, int32_t
   rt.Wr = Wr;
   int32_t *pl = sl.pl;
   u64 *rows = (srows && d <= MEM_SROWS_D) ? srows : sl.rows;  // srows: 2 * MEM_SROWS_D words
-  rt.rows = rows;
-  const int pc = p_cap(d);
   for (int i = lane; i < d; i += 32) pl[i] = a.cs[sb + i];
+  const u64 *wrows = a.enc ? a.wptr[r] : nullptr;
+  if (wrows) {  // rows built before the search (enc.cu)
+    rt.rows = wrows;
+    rt.xr = wrows + (size_t)d * Wr;
+    rt.nX = u;
+    if (rows == srows) {
+      for (int i = lane; i < d * Wr; i += 32) srows[i] = wrows[i];
+      rt.rows = srows;
+    }
+    __syncwarp();
+    return;
+  }
+  rt.rows = rows;
+  rt.xr = sl.xr;
+  const int pc = p_cap(d);
   for (int i = lane; i < d * Wr; i += 32) rows[i] = 0;
   for (int i = lane; i < pc; i += 32) sl.pkey[i] = -1;
   __syncwarp();
@@ -1348,15 +1436,15 @@ __device__ void mem_encode(const BKArgs &a, MemSmem &sm, const Slab &sl, int32_t
 // Walk the subtree under frame 0 of the slab stack (P, X, S already there).
 // Whether one of the nL filtered earlier-neighbour rows contains the chosen
 // set Cs (Wr words in the slab): the leaf's clique is then not maximal.
-__device__ __forceinline__ bool mem_covered(const Slab &sl, int nL, int Wr, const u64 *Cs,
-                                            const u64 *rows) {
+__device__ __forceinline__ bool mem_covered(const Slab &sl, const u64 *xr, int nL, int Wr,
+                                            const u64 *Cs, const u64 *rows) {
   const int lane = (int)lane_id();
   for (int i0 = 0; i0 < nL; i0 += 32) {
     const int i = i0 + lane;
     bool hit = false;
     if (i < nL) {
       const int32_t k = sl.xl[i];
-      const u64 *xrow = k >= 0 ? sl.xr + (size_t)k * Wr : rows + (size_t)(-1 - k) * Wr;
+      const u64 *xrow = k >= 0 ? xr + (size_t)k * Wr : rows + (size_t)(-1 - k) * Wr;
       hit = true;
       for (int w = 0; w < Wr && hit; ++w) hit = (xrow[w] & Cs[w]) == Cs[w];
     }
@@ -1412,7 +1500,8 @@ __device__ __forceinline__ void mem_leaf(const BKArgs &a, const Slab &sl, int32_
 // rows (sl.xo) - the best score |P & row| with the lowest row id (earlier-
 // neighbour rows first).  Returns score + 1 (0: no such row) with the row in
 // *row_out; *elim: one of them covers P.
-__device__ __forceinline__ int mem_outside_pivot(const Slab &sl, const u64 *rows, int nX, int d,
+__device__ __forceinline__ int mem_outside_pivot(const Slab &sl, const u64 *xr, const u64 *rows,
+                                                 int nX, int d,
                                                  int Wr, bool xo, const u64 *S, const u64 *P,
                                                  int pc, bool *elim, const u64 **row_out) {
   const int lane = (int)lane_id();
@@ -1423,7 +1512,7 @@ __device__ __forceinline__ int mem_outside_pivot(const Slab &sl, const u64 *rows
   for (int i = lane; i < total; i += 32) {
     const u64 *row;
     if (i < nX) {
-      row = sl.xr + (size_t)i * Wr;
+      row = xr + (size_t)i * Wr;
     } else {
       const int j = i - nX;
       if (!((sl.xo[j >> 6] >> (j & 63)) & 1ull)) continue;
@@ -1446,7 +1535,7 @@ __device__ __forceinline__ int mem_outside_pivot(const Slab &sl, const u64 *rows
   const int mb = (int)__reduce_max_sync(MCE_FULL, (unsigned)best);
   const uint32_t id = __reduce_min_sync(MCE_FULL, best == mb ? bid : 0xFFFFFFFFu);
   if (mb > 0)
-    *row_out = (int)id < nX ? sl.xr + (size_t)id * Wr : rows + (size_t)((int)id - nX) * Wr;
+    *row_out = (int)id < nX ? xr + (size_t)id * Wr : rows + (size_t)((int)id - nX) * Wr;
   return mb;
 }
 
@@ -1462,7 +1551,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
   const uint32_t lt = (1u << lane) - 1u;
   const int d = rt.d, Wr = rt.Wr, nX = rt.nX;
   const u64 w32 = (u64)((d + 31) >> 5);
-  const u64 *rows = rt.rows;
+  const u64 *rows = rt.rows, *xr = rt.xr;
   const bool share = a.q.hdr != nullptr;
   u64 *F0 = sl.stk;
   // pivot of the start node
@@ -1497,7 +1586,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
     const u64 *orow = nullptr;
     int mb = 0;
     bool elo = false;
-    if constexpr (XP) mb = mem_outside_pivot(sl, rows, nX, d, Wr, L2 && XO, F0 + 3 * Wr, F0, pc, &elo, &orow);
+    if constexpr (XP) mb = mem_outside_pivot(sl, xr, rows, nX, d, Wr, L2 && XO, F0 + 3 * Wr, F0, pc, &elo, &orow);
     if (__any_sync(MCE_FULL, el) || elo || pc == 0) {
       MCE_BD(BD_OTHER);
       return;
@@ -1517,7 +1606,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
       bool has = false;
       if (i < nX) {
         has = true;
-        for (int w = 0; w < Wr && has; ++w) has = (sl.xr[(size_t)i * Wr + w] & S0[w]) == S0[w];
+        for (int w = 0; w < Wr && has; ++w) has = (xr[(size_t)i * Wr + w] & S0[w]) == S0[w];
       }
       const uint32_t m2 = __ballot_sync(MCE_FULL, has);
       if (has) sl.xl[nL + __popc(m2 & lt)] = i;
@@ -1595,7 +1684,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
       nL = 0;
       for (int i0 = 0; i0 < nX; i0 += 32) {
         const int i = i0 + lane;
-        const bool has = i < nX && (sl.xr[(size_t)i * Wr + vw] & vbit);
+        const bool has = i < nX && (xr[(size_t)i * Wr + vw] & vbit);
         const uint32_t m2 = __ballot_sync(MCE_FULL, has);
         if (has) sl.xl[nL + __popc(m2 & lt)] = i;
         nL += __popc(m2);
@@ -1605,7 +1694,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
     if (pc == 0) {
       MCE_BD(BD_MAXIMAL);
       const u64 *Cs = C + 3 * Wr;
-      if (!xnz && !mem_covered(sl, nL, Wr, Cs, rows))
+      if (!xnz && !mem_covered(sl, xr, nL, Wr, Cs, rows))
         mem_leaf<LIST>(a, sl, rt.r, Wr, Cs, s_base + depth, h0, h1, cnt);
       continue;
     }
@@ -1651,7 +1740,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
       u64 *Cl = C + 2 * Wr;
       if (lane < Wr) Cl[lane] = C[3 * Wr + lane] | C[lane];
       __syncwarp();
-      const bool cov = mem_covered(sl, nL, Wr, Cl, rows);
+      const bool cov = mem_covered(sl, xr, nL, Wr, Cl, rows);
       if (XP && cov) continue;
       nodes += (u64)pc;
       if (Budget && a.node_budget && nodes > a.node_budget) {
@@ -1665,7 +1754,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
     int mbo = 0;
     if constexpr (XP) {  // outside rows adjacent to the whole chosen set
       bool elo = false;
-      mbo = mem_outside_pivot(sl, rows, nX, d, Wr, L2 && XO, C + 3 * Wr, C, pc, &elo, &orow);
+      mbo = mem_outside_pivot(sl, xr, rows, nX, d, Wr, L2 && XO, C + 3 * Wr, C, pc, &elo, &orow);
       if (elo) continue;
     }
     if (share && pc >= a.donate_min &&
@@ -1733,7 +1822,7 @@ __device__ __forceinline__ void mem_l2_units(const BKArgs &a, const Slab &sl, co
       for (int i0 = 0; !covered && i0 < nX; i0 += 32) {
         const int i = i0 + lane;
         covered = __any_sync(MCE_FULL,
-                             i < nX && ((sl.xr[(size_t)i * Wr + (v >> 6)] >> (v & 63)) & 1ull));
+                             i < nX && ((rt.xr[(size_t)i * Wr + (v >> 6)] >> (v & 63)) & 1ull));
       }
       if (!covered) mem_leaf<LIST>(a, sl, rt.r, Wr, sl.stk + 3 * Wr, 0, h0, h1, cnt);  // size 2
       continue;

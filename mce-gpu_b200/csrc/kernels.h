@@ -69,10 +69,6 @@ enum RootClass : uint32_t {
 // so hubs with few later neighbours stay in the register engines.
 constexpr int REG_XCAP = 1024;
 constexpr int REG_XCAP_MAX = 16384;
-// Register-class roots with more earlier neighbours than this ("hubs") get
-// their earlier-neighbour rows from a parallel pass before the search, one
-// warp per 32 of them, instead of walking them serially in the root's warp.
-constexpr int HUB_XMIN = 256;
 
 // Per-call summary the device writes and the host reads once.
 struct ShapeInfo {
@@ -82,9 +78,8 @@ struct ShapeInfo {
   uint32_t max_dminus_mem; // over roots of CLS_MEM
   uint32_t max_deg;
   uint32_t max_dminus_reg; // over roots of CLS_R32 and CLS_R64
-  uint32_t hub_cnt;        // register-class roots with d- > HUB_XMIN
-  uint32_t hub_r32;        // ... of them in CLS_R32
-  unsigned long long hub_rows;  // their earlier degrees, each rounded up to 32
+  uint32_t wide_cnt;       // roots of CLS_R64 and CLS_MEM
+  unsigned long long wide_words;  // 64-bit words of their rows (enc.cu)
 };
 
 struct OrientArgs {
@@ -97,8 +92,8 @@ struct OrientArgs {
   ShapeInfo *shape;     // zeroed by the launcher
   const float *cost;    // nullable: per-vertex cost estimate (larger first)
   int sched;
-  int32_t *hub_of;      // nullable, n: index of the vertex in hub_list, or -1
-  int32_t *hub_list;    // n: the hub roots, in no particular order
+  int32_t *wide_list;   // n - v0: the roots wider than 32, in no particular order ...
+  unsigned long long *wide_off;  // ... and where the rows of each begin, in 64-bit words
   int64_t v0 = 0;       // vertices [v0, n) are oriented (a batch part: its range)
   bool keep_shape = false;  // add to the summary of earlier parts instead of zeroing it
   uint32_t *next = nullptr; // two counters (zeroed by the launcher): the launch's row groups
@@ -109,18 +104,24 @@ struct OrientArgs {
 };
 int orient_launch(const OrientArgs &a, cudaStream_t s, int *launches);
 
-// Earlier-neighbour rows of the hub roots (orient's hub_list, cnt of them):
-// off[j] = first row of hub j (rows padded to 32 per hub), rows[k] = the
-// bitmap over the hub's later list of one earlier neighbour's later list.
-// nx[j] = -1: hub j's distinct rows are not known yet (the search sets it).
-// hub_of[list[i]] = i for the cnt hubs of `list` (one hub numbering for
-// hub lists gathered from several parts of a batch).
-int hub_index_launch(const int32_t *list, uint32_t cnt, int32_t *hub_of, cudaStream_t s,
-                     int *launches);
-int hub_rows_launch(const int32_t *rp, const int32_t *split, const int32_t *cs,
-                    const int32_t *hub_list, uint32_t cnt, int64_t total_rows, int64_t *off,
-                    int32_t *nx, unsigned long long *rows, int sms, cudaStream_t s,
-                    int *launches);
+// ---- induced subgraphs before the search (enc.cu) ------------------------------
+struct EncArgs {
+  int64_t n;
+  const int32_t *rp, *split, *cs;
+  const int32_t *roots;      // class-sorted roots
+  const ShapeInfo *shape;    // their cls_off on the device
+  uint32_t *enc;             // m: rows of the roots with d+ <= 32 at their CSR positions
+  unsigned long long **wptr; // n: the rows of each wider root (null: none, see enc_launch)
+  int32_t *nx;               // n: distinct earlier rows once the search has counted them, or -1
+  uint32_t *next;            // root counter, zeroed by the launcher
+};
+// Build the rows of every root of a.roots: vertices [v0, v1), arcs [arc0,
+// arc1).  The wide roots' rows go to wbase (wide_words of the summary; a
+// root whose rows end past wcap words has none and the search encodes it).
+int enc_launch(const EncArgs &a, const int32_t *wide_list, uint32_t wide_cnt,
+               const unsigned long long *woff, unsigned long long *wbase, unsigned long long wcap,
+               uint32_t small_cnt, uint32_t max_dplus, int64_t arc0, int64_t arc1, int64_t v0,
+               int64_t v1, int sms, cudaStream_t s, int *launches);
 
 // Sort roots by key (stable) and compute class offsets.  temp grows on demand.
 int roots_sort(int64_t n, const uint32_t *keys_in, uint32_t *keys_out, const int32_t *vals_in,
@@ -144,10 +145,9 @@ struct BKArgs {
   size_t slab_words;             // u64 words per warp
   int32_t dcap, xcap;            // slab capacities (later degree, x rows)
   int32_t rxcap;                 // register engines' x rows (0: REG_XCAP)
-  const int32_t *hub_of;         // nullable, n: hub index of a root (-1: none) ...
-  const int64_t *hub_off;        // ... its first precomputed earlier-neighbour row ...
-  unsigned long long *hub_rows;  // ... in these rows (hub_rows_launch) ...
-  int32_t *hub_nx;               // ... of which the first hub_nx are distinct once >= 0
+  uint32_t *enc;                 // nullable: the rows built before the search (EncArgs) ...
+  unsigned long long *const *wptr;  // ... of the wider roots ...
+  int32_t *nx;                   // ... and how many earlier rows of a root are distinct
   QueueView q;                   // task queue (q.hdr == nullptr: no sharing)
   int32_t donate_min;            // hand off children with at least this many candidates
   uint32_t donate_after;         // ... once this many nodes of the root/task were walked
@@ -202,12 +202,9 @@ int mlp_adam_launch(float *master, void *wh, float *grad, float *m1, float *m2, 
                     int step, cudaStream_t s);
 // Sort keys by cost: with `cost`, roots with at least cost_min later
 // neighbours take it and the others the degree heuristic.
-// hub_of (nullable, the same n vertices): hub roots sort before the other
-// roots of their class (key bit 27; the cost keeps 27 bits).
 int rekey_launch(int64_t n, uint32_t *keys, const float *cost, const int32_t *rp,
                  const int32_t *split, uint8_t *policy, float heavy_cost, float share_cost,
-                 int sms, cudaStream_t s, int *launches, int cost_min = 0,
-                 const int32_t *hub_of = nullptr);
+                 int sms, cudaStream_t s, int *launches, int cost_min = 0);
 
 // ---- batches ------------------------------------------------------------------
 int batch_rebase_launch(const int32_t *rp_local, const int32_t *col_local,

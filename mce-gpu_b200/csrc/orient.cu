@@ -81,7 +81,7 @@ __device__ int32_t split_long_row(const OrientArgs &a, int32_t v, uint32_t pv, i
 }
 
 // Vertex v with row [b, e) and cntE earlier neighbours: its split point,
-// engine class and sort key, and its entry in the hub list.  Returns the class.
+// engine class and sort key, and a wide root's place for its rows.  Returns the class.
 __device__ __forceinline__ uint32_t finish_vertex(const OrientArgs &a, int32_t v, int32_t b,
                                                   int32_t e, int32_t cntE, uint32_t &dplus,
                                                   uint32_t &dminus) {
@@ -98,15 +98,11 @@ __device__ __forceinline__ uint32_t finish_vertex(const OrientArgs &a, int32_t v
   }
   a.keys_in[v] = key;
   a.vals_in[v] = v;
-  if (a.hub_of) {
-    int32_t hi = -1;
-    if ((cls == CLS_R32 || cls == CLS_R64) && dminus > (uint32_t)HUB_XMIN) {
-      hi = (int32_t)atomicAdd(&a.shape->hub_cnt, 1u);
-      a.hub_list[hi] = v;
-      atomicAdd(&a.shape->hub_rows, (unsigned long long)((dminus + 31u) & ~31u));
-      if (cls == CLS_R32) atomicAdd(&a.shape->hub_r32, 1u);
-    }
-    a.hub_of[v] = hi;
+  if (cls == CLS_R64 || cls == CLS_MEM) {
+    const uint32_t k = atomicAdd(&a.shape->wide_cnt, 1u);
+    a.wide_list[k] = v;
+    a.wide_off[k] = atomicAdd(&a.shape->wide_words,
+                              (unsigned long long)(dplus + dminus) * ((dplus + 63u) >> 6));
   }
   return cls;
 }
