@@ -113,6 +113,27 @@ __global__ void __launch_bounds__(REG_BLOCK, (NR == 1 && sizeof(Word) == 4) ? 6 
       }
     }
   }
+  if constexpr (NR == 1 && sizeof(Word) == 4 && EV == 0 && !LIST && !XP && !OPS && !SPLIT &&
+                !STAGE && !L2) {
+    // frames the lane engine handed over (a.resume)
+    const uint32_t frames = a.resume ? min(*a.resume_count, a.resume_cap) : 0u;
+    while (frames) {
+      uint32_t i = 0;
+      if (lane == 0) i = atomicAdd(a.resume_next, 1u);
+      i = __shfl_sync(MCE_FULL, i, 0);
+      if (i >= frames) break;
+      const uint32_t *f = a.resume + (size_t)i * RESUME_WORDS;
+      const int32_t r = (int32_t)f[0];
+      if (r < 0) continue;  // a slot that was given up
+      if (r != rt.r) reg_encode<Word, NR, STAGE>(a, sm, sl, r, rt, false);
+      u64 nd = 0, cnt = 0, op = 0;
+      reg_tree<Word, NR, false, EV, LIST, XP, OPS, false>(a, sm, sl, rt, f[1], f[2], f[3], h0, h1,
+                                                          nd, cnt, bd, &op, 0, 1, (Word)0, true,
+                                                          f[4], f[5]);
+      nodes += nd;
+      root_done(a, r, nd, cnt);
+    }
+  }
   if (share) {
     root_phase_done(a.q);
     u64 t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
@@ -134,7 +155,7 @@ __global__ void __launch_bounds__(REG_BLOCK, (NR == 1 && sizeof(Word) == 4) ? 6 
           const Word S = (Word)__shfl_sync(MCE_FULL, t3, 3);
           const Word XO = L2 ? (Word)__shfl_sync(MCE_FULL, t4, 4) : (Word)0;  // L2 unit's outside rows
           MCE_BD(BD_ENCODE);
-          if (r != rt.r) reg_encode<Word, NR, STAGE>(a, sm, sl, r, rt);
+          if (r != rt.r) reg_encode<Word, NR, STAGE>(a, sm, sl, r, rt, false);
           u64 nd = 0, cnt = 0, op = 0;
           reg_tree<Word, NR, false, EV, LIST, XP, OPS, false, L2>(a, sm, sl, rt, P, X, S, h0, h1, nd,
                                                                   cnt, bd, &op, 0, 1, XO);

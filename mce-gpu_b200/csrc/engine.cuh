@@ -367,14 +367,14 @@ struct RegRoot {
 // A root whose rows were built before the search: at its CSR positions
 // (enc, 32-bit words) or in its region (wrows).  The distinct non-empty
 // earlier rows go to sl.xr in list order; more than 32 of them are
-// deduplicated once: the first warp to load the root writes the distinct ones
-// back over the built ones and publishes their number (nx), so the warps that
-// take its subtrees later only copy them.
+// deduplicated once: the warp that searches the root (publish) writes the
+// distinct ones back over the built ones and publishes their number (nx), so
+// the warps that take its subtrees later only copy them.
 template <typename Word, int NR>
 __device__ __forceinline__ void reg_load(const BKArgs &a, RegSmem<Word, NR> &sm,
                                          const RegSlab<Word> &sl, int32_t r, int32_t ub, int u,
                                          int32_t sb, int d, uint32_t *enc,
-                                         unsigned long long *wrows, RegRoot<Word> &rt) {
+                                         unsigned long long *wrows, bool publish, RegRoot<Word> &rt) {
   const int lane = (int)lane_id();
   const uint32_t lt = (1u << lane) - 1u;
   auto earlier = [&](int i) -> Word {  // from L2: another warp may have rewritten them
@@ -437,9 +437,9 @@ __device__ __forceinline__ void reg_load(const BKArgs &a, RegSmem<Word, NR> &sm,
     __syncwarp();
   }
   rt.nX = nX;
-  // with several warps per root two of them may load it at once, so then the
-  // rows stay as built and every warp deduplicates them itself
-  if (a.parts <= 1) {
+  // where several warps may load the root at once (parts of it, frames handed
+  // over by the lane engine) the rows stay as built and each deduplicates them
+  if (publish && a.parts <= 1) {
     for (int i = lane; i < nX; i += 32) {
       if (enc)
         enc[ub + i] = (uint32_t)sl.xr[i];
@@ -455,7 +455,7 @@ __device__ __forceinline__ void reg_load(const BKArgs &a, RegSmem<Word, NR> &sm,
 // STAGE: the lists are staged in shared memory by bulk copies (*stg).
 template <typename Word, int NR, bool STAGE = false>
 __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<Word> &sl,
-                           int32_t r, RegRoot<Word> &rt) {
+                           int32_t r, RegRoot<Word> &rt, bool publish = true) {
   using O = WOps<Word>;
   const int lane = (int)lane_id();
   const uint32_t lt = (1u << lane) - 1u;
@@ -484,7 +484,7 @@ __device__ void reg_encode(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab
       wrows = a.wptr[r];
   }
   if (enc || wrows) {
-    reg_load<Word, NR>(a, sm, sl, r, ub, u, sb, d, enc, wrows, rt);
+    reg_load<Word, NR>(a, sm, sl, r, ub, u, sb, d, enc, wrows, publish, rt);
     return;
   }
 
@@ -760,12 +760,15 @@ __device__ __forceinline__ void reg_emit(const BKArgs &a, const RegSmem<Word, NR
 // SPLIT: the variant for several warps per root (part / parts below).
 // L2: the variant that carries an L2 unit's outside rows (XO); the others
 // ignore XO.
+// resume (a frame of the lane engine): the node's pivot is chosen already, RB
+// its branches left to walk and RL its settled leaves.
 template <typename Word, int NR, bool Budget = false, int EV = 0, bool LIST = false,
           bool XP = false, bool OPS = false, bool SPLIT = false, bool L2 = false>
 __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<Word> &sl,
                          const RegRoot<Word> &rt, Word P, Word X, Word S, u64 &h0, u64 &h1,
                          u64 &nodes, u64 &cnt, Bd *bd = nullptr, u64 *ops = nullptr,
-                         int part = 0, int parts = 1, Word XO = 0) {
+                         int part = 0, int parts = 1, Word XO = 0, bool resume = false,
+                         Word RB = 0, Word RL = 0) {
   using O = WOps<Word>;
   const u64 w32 = (u64)((rt.d + 31) >> 5);
   MCE_BD(BD_PIVOT);
@@ -780,7 +783,7 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
   // root is adjacent to all of it.  Same nodes and count, no walk.
   if constexpr (!XP && !OPS) {
     const int d = rt.d;
-    if (S == 0 && X == 0 && P == O::low(d) && d > 0) {
+    if (S == 0 && X == 0 && P == O::low(d) && d > 0 && !resume) {
       bool full = lane >= d || ((r0 | O::bit(lane)) & P) == P;
       if constexpr (NR == 2) full = full && (lane + 32 >= d || ((r1 | O::bit(lane + 32)) & P) == P);
       if (__all_sync(MCE_FULL, full)) {
@@ -855,7 +858,7 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
   Word start_row = 0;
   bool start_out = false;
   bool iso0 = false, iso1 = false;  // this lane's candidate has no neighbour in P
-  {
+  if (!resume) {
     const Word cand = P | X;
     const int pc = O::popc(P);
     if constexpr (OPS)
@@ -899,6 +902,7 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
   MCE_BD(BD_SETS);
   // apply_pivot_to_first_level (:204-216) / apply_pivot_to_next_level (:218-239)
   Word B = P & ~(start_out ? start_row : row_of<Word, NR>(r0, r1, 127 - (start_k & 127)));
+  if (resume) B = RB;
   int depth = 0, recheck = 0, b0 = 0;  // b0: first-level branches passed
   bool want = false;
   // Leaves in bulk: a branch u of the node (Pn, Xn, Sn) with no neighbour in
@@ -969,7 +973,9 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
     return L;
   };
   if constexpr (kBulk) {
-    if (!(SPLIT && parts > 1)) {  // a split root's first level keeps its order
+    if (resume) {
+      Lp = RL;
+    } else if (!(SPLIT && parts > 1)) {  // a split root's first level keeps its order
       Lp = take_leaves(B, P, X, S);
       B &= ~Lp;
     }

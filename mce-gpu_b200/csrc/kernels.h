@@ -148,6 +148,10 @@ struct BKArgs {
   uint32_t *enc;                 // nullable: the rows built before the search (EncArgs) ...
   unsigned long long *const *wptr;  // ... of the wider roots ...
   int32_t *nx;                   // ... and how many earlier rows of a root are distinct
+  const uint32_t *resume;        // nullable: frames the lane engine handed over (RESUME_WORDS) ...
+  const uint32_t *resume_count;  // ... their number (may pass resume_cap) ...
+  uint32_t *resume_next;         // ... and the next one to take
+  uint32_t resume_cap;
   QueueView q;                   // task queue (q.hdr == nullptr: no sharing)
   int32_t donate_min;            // hand off children with at least this many candidates
   uint32_t donate_after;         // ... once this many nodes of the root/task were walked
@@ -172,6 +176,35 @@ struct BKArgs {
   unsigned long long *ops;       // ... into *ops ...
   unsigned long long *root_ops;  // ... and per root (nullable [n])
 };
+
+// ---- lane engine (lane.cu) -----------------------------------------------------
+// A frame handed to the warp engine: root, P, X, chosen set, branch set,
+// settled leaves (a slot that was given up has root 0xFFFFFFFF).
+constexpr int RESUME_WORDS = 6;
+constexpr uint32_t RESUME_CAP = 1u << 18;
+// Counters of one search of the lane engine, zeroed by lane_launch.
+struct LaneCtl {
+  uint32_t next[2];        // next root of each launch
+  uint32_t mid_count;      // roots of the second launch
+  uint32_t resume_count, resume_next;
+  ShapeInfo rest;          // the warp engine's: rest.cls_off[1] roots
+};
+struct LaneArgs {
+  const int32_t *rp, *split, *roots;
+  const uint32_t *count;   // number of roots
+  uint32_t *next;
+  const uint32_t *enc;     // the roots' rows (EncArgs)
+  unsigned long long *hist, *nodes, *root_nodes, *root_count, *graph_count;
+  const int32_t *graph_of;
+  int32_t *mid, *rest;     // roots left to the second launch / to the warp engine ...
+  uint32_t *mid_count, *rest_count;
+  uint32_t *resume, *resume_count;  // ... and frames (RESUME_CAP of them)
+};
+// Searches the roots of a.roots (*count of them, all with d+ <= 32) that suit
+// a lane; the others go to `rest` and are the warp engine's, with
+// ctl->rest as its summary and the frames of `resume`.
+int lane_launch(const BKArgs &b, const uint32_t *count, int32_t *mid, int32_t *rest,
+                uint32_t *resume, LaneCtl *ctl, int sms, cudaStream_t s, int *launches);
 
 // Launch the engine of one class.  warps_out: number of warps launched (slab sizing).
 int bk_warps_for_class(int cls, int sms, int wide_blocks, int *warps, int *block, int *smem);
