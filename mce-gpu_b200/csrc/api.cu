@@ -65,6 +65,7 @@ struct mce_graph {
   unsigned long long *wide_off = nullptr;
   unsigned long long *wide[1 + MAX_BATCH_PARTS] = {nullptr};  // the wide roots' rows, indexed as enc_next
   uint64_t wide_cap[1 + MAX_BATCH_PARTS] = {0};               // ... and the words they hold
+  bool wide_all = true;  // every wide root of the current call has its rows
   ShapeInfo *shape = nullptr;
   void *sort_tmp = nullptr;
   size_t sort_tmp_bytes = 0;
@@ -120,7 +121,7 @@ struct mce_graph {
   size_t part_tmp_bytes[MAX_BATCH_PARTS] = {0};
   // search launches captured as a CUDA graph, replayed while the key matches
   cudaGraphExec_t search_exec = nullptr;
-  unsigned char search_key[320] = {0};
+  unsigned char search_key[512] = {0};
 };
 
 namespace {
@@ -136,6 +137,7 @@ constexpr uint32_t DEFAULT_SOLO_MAX = 0;     // measured slower than grid-wide r
 constexpr uint32_t DEFAULT_DONATE_AFTER = 256;  // the reference's SZTH (mce/parameter.cuh:5)
 
 constexpr int MAX_PARTS = MAX_BATCH_PARTS;
+constexpr int MEM_THREADS = 128;  // threads per block of the wide class's launches
 
 void free_graph_bufs(mce_graph *g) {
   dfree(g->rp); dfree(g->col); dfree(g->cs); dfree(g->split);
@@ -468,6 +470,7 @@ int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const Shape
       (void)cudaGetLastError();  // too large for what is left: try half
     }
   }
+  if (sh.wide_words > g->wide_cap[i]) g->wide_all = false;
   EncArgs ea;
   ea.n = g->n;
   ea.rp = g->rp;
@@ -482,6 +485,36 @@ int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const Shape
   return enc_launch(ea, wide_list, sh.wide_cnt, wide_off, g->wide[i],
                     std::min<uint64_t>(want, g->wide_cap[i]), sh.cls_cnt[CLS_R32], sh.max_dplus,
                     arc0, arc1, v0, v1, g->sms, s, launches);
+}
+
+// The launches of the wide class, widest roots first: bk_mem_kernel (W = 0)
+// above 256 later neighbours, the engines of 256 and of 128 (wide.cu) below,
+// for counts without logs, units or parts whose roots all have their rows;
+// otherwise bk_mem_kernel for all of them.
+struct WideLaunch {
+  int W, d_lo, fetch, grid, block;
+  size_t slab_words;
+};
+
+int plan_wide(const mce_graph *g, const mce_opts_t &o, int parts, bool list, int max_dplus, int xcap,
+              std::vector<WideLaunch> *out) {
+  int rc, warps = 0, block = 0, smem = 0;
+  const bool xp = o.x_pivot || o.induced == MCE_INDUCED_PX;
+  const bool fast = !list && !o.warp_log && !o.count_ops && o.level != MCE_LEVEL_L2 && parts <= 1 &&
+                    g->wide_all;
+  out->clear();
+  if (!fast || max_dplus > 256) {
+    if ((rc = bk_warps_for_class(CLS_MEM, g->sms, o.wide_blocks, &warps, &block, &smem))) return rc;
+    out->push_back({0, fast ? 256 : 0, CLS_MEM, warps / (block / 32), block,
+                    bk_slab_words(CLS_MEM, max_dplus, xcap)});
+  }
+  for (int W = 4; fast && W >= 2; W -= 2) {
+    if (W == 4 && max_dplus <= 128) continue;
+    WideLaunch l{W, W == 4 ? 128 : 0, W == 4 ? 5 : 6, 0, 128, 0};
+    if ((rc = wide_plan(W, xp, g->sms, xcap, &l.grid, &l.slab_words))) return rc;
+    out->push_back(l);
+  }
+  return MCE_OK;
 }
 
 // Whether the 32-bit class of a search starts in the lane engine: a plain
@@ -902,6 +935,7 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   if ((rc = read_shape(g, s))) return rc;
   const ShapeInfo &sh = g->shape_h;
   if (sh.cls_cnt[CLS_BIG]) return MCE_ELIMIT;
+  g->wide_all = true;
   if ((rc = run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0, g->n, s,
                     &launches)))
     return rc;
@@ -924,7 +958,20 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     const int af = o.bucket_donate_after[c] ? o.bucket_donate_after[c] : o.donate_after;
     dafter[c] = af > 0 ? af : (int)DEFAULT_DONATE_AFTER;
   }
-  for (int c = CLS_R32; c <= CLS_MEM; ++c) {
+  std::vector<WideLaunch> wl;
+  if (sh.cls_cnt[CLS_MEM]) {
+    if ((rc = plan_wide(g, o, parts[CLS_MEM], lc != nullptr, dcap, xcap, &wl))) return rc;
+    block[CLS_MEM] = MEM_THREADS;
+    for (WideLaunch &l : wl) {
+      if (!share) {  // never more warps than units of work
+        const int64_t units = (int64_t)sh.cls_cnt[CLS_MEM] * parts[CLS_MEM];
+        l.grid = (int)std::min<int64_t>(l.grid, (units + 3) / 4);
+      }
+      grid[CLS_MEM] = std::max(grid[CLS_MEM], l.grid);
+      slab_need = std::max(slab_need, (size_t)l.grid * 4 * l.slab_words * 8);
+    }
+  }
+  for (int c = CLS_R32; c <= CLS_R64; ++c) {
     if (!sh.cls_cnt[c]) continue;
     int warps = 0;
     if ((rc = bk_warps_for_class(c, g->sms, o.wide_blocks, &warps, &block[c], &smem[c]))) return rc;
@@ -1009,6 +1056,7 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   // opts.cuda_graph it is captured once and replayed.
   struct SearchKey {
     int grid[NCLS], block[NCLS];
+    int wide[3][3];
     int dcap, xcap, rxcap, wbits, share, log, wide8, level2, xpiv, ops, stage, lanes;
     int parts[NCLS], dmin[NCLS], dafter[NCLS];
     uint64_t wlimit;
@@ -1021,6 +1069,11 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     key.grid[c] = grid[c];
     key.block[c] = block[c];
     key.q[c] = qv[c].hdr;
+  }
+  for (size_t i = 0; i < wl.size(); ++i) {
+    key.wide[i][0] = wl[i].W;
+    key.wide[i][1] = wl[i].d_lo;
+    key.wide[i][2] = wl[i].grid;
   }
   key.dcap = dcap;
   key.xcap = xcap;
@@ -1091,6 +1144,19 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
       a.q = share ? qv[c] : QueueView();
       a.warp_log = o.warp_log ? g->wlog + WLOG_WORDS * wlog_base[c] : nullptr;
       a.warp_cycles = o.warp_log == 2 ? 1 : 0;
+      if (c == CLS_MEM) {
+        MCE_CUDA(mark(g->cls_ev[c][0]));
+        for (const WideLaunch &l : wl) {
+          a.slab_words = l.slab_words;
+          a.d_lo = l.d_lo;
+          if (share && (r2 = queue_launch_init(a.q, s, &launches))) return r2;
+          if ((r2 = l.W ? wide_launch(l.W, a.x_pivot != 0, a, l.d_lo, l.fetch, l.grid, s, &launches)
+                        : bk_launch(c, wbits, a, l.grid, l.block, 0, s, &launches)))
+            return r2;
+        }
+        MCE_CUDA(mark(g->cls_ev[c][1]));
+        continue;
+      }
       if (share && (r2 = queue_launch_init(a.q, s, &launches))) return r2;
       MCE_CUDA(mark(g->cls_ev[c][0]));
       if (c == CLS_R32 && lanes &&
@@ -1129,7 +1195,8 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
       std::memcpy(g->search_key, &key, sizeof(key));
     }
     MCE_CUDA(cudaGraphLaunch(g->search_exec, s));
-    for (int c = CLS_R32; c <= CLS_MEM; ++c) launches += grid[c] ? (share ? 2 : 1) : 0;
+    for (int c = CLS_R32; c <= CLS_R64; ++c) launches += grid[c] ? (share ? 2 : 1) : 0;
+    launches += (int)wl.size() * (share ? 2 : 1);
     if (lanes) launches += 2;
   } else {
     if ((rc = record())) return rc;
@@ -1456,6 +1523,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
   // search once those are done: no stream then waits on an event at the
   // head of a hardware queue that other streams share.
   if (!g->part_sdone) MCE_CUDA(cudaEventCreateWithFlags(&g->part_sdone, cudaEventDisableTiming));
+  g->wide_all = true;
   int na = 0, nb = 0, ns = 0;
   auto ready = [&](cudaEvent_t e, int *bad) {
     const cudaError_t q = cudaEventQuery(e);
@@ -1511,6 +1579,12 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       const int cls_of[2] = {CLS_R64, CLS_MEM};
       int grid[2] = {0}, block[2] = {0}, smem[2] = {0}, pc[2] = {1, 1}, dm[2] = {0}, da[2] = {0};
       QueueView qv[2];
+      std::vector<WideLaunch> wl;
+      if (ncls[1] > 0 && (rc = plan_wide(g, o, o.bucket_warps_per_root[CLS_MEM]
+                                                   ? o.bucket_warps_per_root[CLS_MEM]
+                                                   : o.warps_per_root,
+                                         false, dcap, xcap, &wl)))
+        return finish(rc);
       for (int i = 0; i < 2; ++i)
         if (ncls[i] > 0 && (rc = plan(cls_of[i], ncls[i], dcap, xcap, rxcap, &grid[i], &block[i],
                                       &smem[i], &pc[i], &dm[i], &da[i], &qv[i])))
@@ -1520,10 +1594,34 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       a.roots = dlist;
       a.shape = sh_final;
       a.fetch = g->part_fetch + 8 * MAX_PARTS;
-      for (int i : {1, 0})  // wide, then 64-bit
-        if (ncls[i] > 0 && (rc = run_class(cls_of[i], a, grid[i], block[i], smem[i], pc[i], dm[i],
-                                           da[i], qv[i], dcap, xcap, rxcap)))
+      for (const WideLaunch &l : wl) {  // wide, then 64-bit
+        const size_t need = (size_t)l.grid * 4 * l.slab_words * 8;
+        if (need > g->slab_bytes) {  // earlier searches of the call keep the old slab
+          if (g->slab) retired.push_back(g->slab);
+          g->slab = nullptr;
+          g->slab_bytes = 0;
+          if ((rc = dalloc((char **)&g->slab, need))) return finish(rc);
+          g->slab_bytes = need;
+        }
+        if (!l.W) {
+          a.d_lo = l.d_lo;
+          if ((rc = run_class(CLS_MEM, a, l.grid, l.block, 0, pc[1], dm[1], da[1], qv[1], dcap, xcap,
+                              rxcap)))
+            return finish(rc);
+          continue;
+        }
+        a.slab = g->slab;
+        a.slab_words = l.slab_words;
+        a.donate_min = dm[1];
+        a.donate_after = (uint32_t)da[1];
+        a.q = share_q ? qv[1] : QueueView();
+        if ((share_q && (rc = queue_launch_init(a.q, s, &launches))) ||
+            (rc = wide_launch(l.W, a.x_pivot != 0, a, l.d_lo, l.fetch, l.grid, s, &launches)))
           return finish(rc);
+      }
+      if (ncls[0] > 0 && (rc = run_class(CLS_R64, a, grid[0], block[0], smem[0], pc[0], dm[0], da[0],
+                                         qv[0], dcap, xcap, rxcap)))
+        return finish(rc);
     }
   }
   trace_mark(g, s, "final");

@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(MEM_BLOCK, MINB) bk_mem_kernel(BKArgs a, int c
     if (i0 >= units) break;
     const int32_t r = a.roots[beg + i0 / parts];
     MCE_BD(BD_ENCODE);
+    if (a.d_lo && a.rp[r + 1] - a.split[r] <= a.d_lo) continue;
     if (parts == 1 || r != rt.r) mem_encode(a, sm, sl, r, rt, srows);
     MCE_BD(BD_OTHER);
     if (rt.d == 0) continue;

@@ -161,6 +161,7 @@ struct BKArgs {
   unsigned long long *warp_log;  // nullable: per warp of the launch {SM id, tree nodes, donations,
                                  // cycles per phase[7]}
   int32_t warp_cycles;           // 1: also the per-phase cycle breakdown
+  int32_t d_lo;                  // bk_mem_kernel: roots with d+ <= d_lo are another launch's
   int32_t wide8;                 // 1: the wide engine's 8-blocks-per-SM variant
   int32_t level2;                // 1 (-p l2): edge-rooted units, offered to idle warps at once
   const uint32_t *prio;          // peel priorities (the degeneracy order of the L2 units)
@@ -205,6 +206,12 @@ struct LaneArgs {
 // ctl->rest as its summary and the frames of `resume`.
 int lane_launch(const BKArgs &b, const uint32_t *count, int32_t *mid, int32_t *rest,
                 uint32_t *resume, LaneCtl *ctl, int sms, cudaStream_t s, int *launches);
+
+// ---- wide engine of up to 64 W later neighbours, W = 2 or 4 (wide.cu) ------------
+int wide_plan(int W, bool xp, int sms, int xcap, int *grid, size_t *slab_words);
+// The roots of CLS_MEM with d+ in (d_lo, 64 W]; fetch: the launch's root counter.
+int wide_launch(int W, bool xp, const BKArgs &a, int d_lo, int fetch, int grid, cudaStream_t s,
+                int *launches);
 
 // Launch the engine of one class.  warps_out: number of warps launched (slab sizing).
 int bk_warps_for_class(int cls, int sms, int wide_blocks, int *warps, int *block, int *smem);
