@@ -25,7 +25,9 @@ int graph_adopt(int32_t device, int64_t n, int64_t m, struct ::mce_graph **out, 
 namespace {
 
 constexpr uint32_t BEL_RANGE = 1u, BEL_ORDER = 2u, BEL_LOOP = 4u, BEL_DST = 8u;
-constexpr int64_t BEL_CHUNK = 1 << 21;  // records per staging buffer (48 MiB)
+// Records per staging buffer (3 MiB): pinning costs more per byte than reading
+// does, and a file of one chunk would be read, copied and decoded in turn.
+constexpr int64_t BEL_CHUNK = 1 << 17;
 
 __global__ void bel_decode_kernel(const unsigned long long *__restrict__ raw, int64_t count,
                                   int64_t base, int32_t *__restrict__ src,
