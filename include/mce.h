@@ -99,7 +99,7 @@ typedef struct mce_opts {
                                search trees are not                          */
   int32_t peel_solo_max;    /* 0 = default (off); < 0 = off; > 0: frontiers of at most
                                this many vertices are peeled by one block           */
-  int32_t donate_after;     /* 0 = default (256): a warp shares subtrees of a
+  int32_t donate_after;     /* 0 = default (16): a warp shares subtrees of a
                                root only after walking this many of its nodes */
   int32_t cuda_graph;       /* 1 = capture the search launches in a CUDA graph
                                once and replay it (default for batches)      */

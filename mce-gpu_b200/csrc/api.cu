@@ -136,7 +136,11 @@ static_assert(sizeof(QueueHdr) <= QUEUE_HDR, "queue header");
 constexpr int DEFAULT_DONATE_MIN = 10;
 constexpr int64_t BATCH_PART_MIN_ARCS = 1 << 20;  // mce_batch_count_host: smaller batches in one part
 constexpr uint32_t DEFAULT_SOLO_MAX = 0;     // measured slower than grid-wide rounds
-constexpr uint32_t DEFAULT_DONATE_AFTER = 256;  // the reference's SZTH (mce/parameter.cuh:5)
+// Nodes of a root or task before its subtrees are shared.  16 against 256 (the
+// best while a push cost the whole device 0.9 us): search of R-MAT 12 with -i
+// px 1.80 against 4.67 ms, of R-MAT 13 8.5 and 9.4, of BA n = 1e6 1.72 and
+// 2.05, of 1,024 Chung-Lu graphs 6.66 and 6.87; 64 lies between.
+constexpr uint32_t DEFAULT_DONATE_AFTER = 16;
 
 constexpr int MAX_PARTS = MAX_BATCH_PARTS;
 constexpr int MEM_THREADS = 128;  // threads per block of the wide class's launches

@@ -48,7 +48,7 @@ struct Knobs {
 Knobs resolved(const mce_opts_t &o) {
   Knobs k;
   k.worker_list = o.worker_list ? o.worker_list : MCE_WL_ON;
-  k.donate_after = o.donate_after > 0 ? o.donate_after : 256;
+  k.donate_after = o.donate_after > 0 ? o.donate_after : 16;
   k.donate_threshold = o.donate_threshold > 0 ? o.donate_threshold : 10;
   k.bitmap_width = o.bitmap_width ? o.bitmap_width : 32;
   k.peel_solo_max = o.peel_solo_max > 0 ? o.peel_solo_max : -1;
@@ -242,7 +242,7 @@ int tune(const char *key, const mce_opts_t &base, const char *table_path, int32_
     std::vector<int32_t> values;
   };
   const Axis axes[] = {
-      {&Knobs::donate_after, {64, 256, 1024}},
+      {&Knobs::donate_after, {16, 64, 256}},
       {&Knobs::donate_threshold, {6, 10, 16}},
       {&Knobs::bitmap_width, {32, 64}},
       {&Knobs::peel_solo_max, {-1, 64}},
@@ -292,7 +292,7 @@ int tune(const char *key, const mce_opts_t &base, const char *table_path, int32_
     };
     const BAxis baxes[] = {{&Bucket::warps, {1, 2, 4}, false},
                            {&Bucket::threshold, {6, 10, 16}, true},
-                           {&Bucket::after, {64, 256, 1024}, true}};
+                           {&Bucket::after, {16, 64, 256}, true}};
     for (const BAxis &ax : baxes) {
       if (ax.donation && !wl) continue;
       Bucket best = b;
