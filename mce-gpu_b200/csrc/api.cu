@@ -493,6 +493,8 @@ int run_parts(mce_graph *g, cudaStream_t s, int *launches, const BatchCtx *bc, i
 // whole graph) before its search.  The wide roots' rows are bounded by
 // WIDE_BYTES and by what the device has left: the search encodes the rest.
 constexpr uint64_t WIDE_BYTES = 32ull << 30;
+constexpr uint32_t ROWS_MIN_ROOTS = 16384, ROWS_MAX_EARLIER = 256;
+constexpr uint32_t SHARE_MIN_LATER = 16;
 
 int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const ShapeInfo *shape_dev,
             int i, const int32_t *wide_list, const unsigned long long *wide_off, int64_t arc0,
@@ -968,11 +970,18 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   const ShapeInfo &sh = g->shape_h;
   if (sh.cls_cnt[CLS_BIG]) return MCE_ELIMIT;
   g->wide_all = true;
-  if ((rc = run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0, g->n, s,
-                    &launches)))
+  // A few thousand narrow roots without hubs are encoded by the search's own
+  // warps: building their rows first would only add launches (ER n = 200 254
+  // against 236 us, n = 10,000 461 against 441 us a call).
+  const bool rows = sh.wide_cnt > 0 || sh.cls_cnt[CLS_R32] >= ROWS_MIN_ROOTS ||
+                    sh.max_dminus_reg > ROWS_MAX_EARLIER;
+  if (rows && (rc = run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0,
+                            g->n, s, &launches)))
     return rc;
   // search scratch
-  const bool share = o.worker_list != MCE_WL_OFF;
+  // Trees over at most 16 later neighbours have a few hundred nodes: nothing
+  // to share, and no idle warps to launch for it.
+  const bool share = o.worker_list != MCE_WL_OFF && sh.max_dplus > SHARE_MIN_LATER;
   int grid[NCLS] = {0}, block[NCLS] = {0}, smem[NCLS] = {0};
   const int dcap = (int)(sh.max_dplus > 0 ? sh.max_dplus : 1);
   const int xcap = (int)(sh.max_dminus_mem > 0 ? sh.max_dminus_mem : 1);
@@ -1055,7 +1064,7 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   a.dcap = dcap;
   a.xcap = xcap;
   a.rxcap = rxcap;
-  a.enc = g->enc;
+  a.enc = rows ? g->enc : nullptr;
   a.wptr = g->wptr;
   a.nx = g->nx;
   a.donate_min = dmin[CLS_R32];  // set per class at each launch below
