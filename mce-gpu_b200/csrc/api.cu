@@ -565,7 +565,7 @@ int plan_wide(const mce_graph *g, const mce_opts_t &o, int parts, bool list, int
 // warps.  32-bit class with lanes and without: 2.86 M roots of 1,024 Chung-Lu
 // graphs 2.40 and 3.98 ms, 0.71 M of 256 graphs 1.16 and 1.24, 1.00 M of BA
 // n = 1e6 0.30 and 0.78, 40,000 of 64 graphs 0.39 and 0.17.
-constexpr uint32_t LANE_MIN_ROOTS = 1000000;
+constexpr uint32_t LANE_MIN_ROOTS = 400000;
 
 bool use_lanes(const mce_opts_t &o, uint32_t roots, int parts, bool list) {
   return roots >= LANE_MIN_ROOTS && o.bitmap_width != 64 && o.level != MCE_LEVEL_L2 &&
