@@ -113,7 +113,8 @@ typedef struct mce_opts {
                                and donations; 2 = also its clock cycles per
                                phase (read both with mce_warp_log)           */
   int32_t wide_blocks;      /* 0 = default (4): blocks per SM of the wide
-                               engine (d+ > 64); 8 = its 64-register variant */
+                               engine where its general kernel runs (d+ > 256,
+                               logs, listing, L2); 8 = its 64-register variant */
   int32_t wait_limit_ms;    /* 0 = default (30 s): a search warp waiting for
                                subtrees gives up after this long without
                                progress anywhere and the call returns
@@ -133,8 +134,9 @@ typedef struct mce_opts {
   int32_t bucket_donate_threshold[3];
   int32_t bucket_donate_after[3];
   int32_t stage_lists;      /* 1 = the 32-bit engine (d+ <= 32, one warp per
-                               root, IP) copies each group of later lists it
-                               encodes into shared memory with 1-D bulk
+                               root, IP) encodes its roots of at most 256 earlier
+                               neighbours itself and copies each group of later
+                               lists into shared memory with 1-D bulk
                                copies (16-byte windows, one mbarrier per
                                warp) and reads them there; groups that do not
                                fit 2 KB are read from global memory         */
@@ -366,17 +368,16 @@ int mce_batch_count(mce_batch_t b, const mce_opts_t *opts, uint64_t *per_graph_t
                     uint64_t *total, uint64_t *hist, mce_stats_t *stats);
 
 /* mce_batch_reload followed by mce_batch_count in one call, for a batch in
- * host memory: batches of 2^20 arcs or more are copied in up to six parts
- * of whole graphs on a stream of the handle's own, and each part is rebased,
- * peeled, oriented and - for counts in plain or degree order without
- * per-root or per-warp logs - its roots with at most 32 later and 256
- * earlier neighbours are searched while the next parts are still being
- * copied (parts of 2, 4, 7, 11, 16 and 24 64ths of the arcs): the host
- * enqueues a part's rebase and peel once its copy has landed, its
- * orientation once the search of the part before it has ended, and its
- * search once it is oriented; the other roots of every part (hub roots,
- * wider bitmaps) follow in one search.  In the other modes one search over
- * the whole batch follows.
+ * host memory: batches of 2^20 arcs or more are copied in parts of whole
+ * graphs on a stream of the handle's own, and each part is rebased, peeled,
+ * oriented and - for counts in plain or degree order without per-root or
+ * per-warp logs, in three parts of 6, 16 and 42 64ths of the arcs - its roots
+ * with at most 32 later neighbours are searched while the next parts are still
+ * being copied: the host enqueues a part's rebase and peel once its copy has
+ * landed, its orientation once the search of the part before it has ended, and
+ * its search once it is oriented; the wider roots of every part follow in one
+ * search.  In the other modes there are six parts and one search over the
+ * whole batch follows.
  * Same results as the two calls.  Pinned host memory lets the copies
  * overlap.  In the part-by-part mode stats->peel_ms is the time until the
  * first part is ready, orient_ms 0 and count_ms the rest.  With the

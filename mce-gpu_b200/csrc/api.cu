@@ -2013,23 +2013,24 @@ int mce_batch_count_host(mce_batch_t b, const int32_t *row_ptr, const int32_t *c
   const int32_t G = num_graphs;
   const int64_t *vo = vtx_offsets, *ao = arc_offsets;
   // Parts of whole graphs; small batches in one.  When the parts are
-  // searched as they arrive, they grow (2, 4, 7, 11, 16 and 24 64ths of the
-  // arcs): the first search starts after a short copy, and since the copy
-  // moves arcs faster than the narrow roots are searched, each part lands
-  // before the search stream reaches it; parts growing 2x per step left the
-  // stream waiting for the last ones, and 3, 5, 8, 12, 16, 20 measured
-  // 0.3 ms slower end to end.  Otherwise they are equal.
+  // searched as they arrive, three of them grow (6, 16 and 42 64ths of the
+  // arcs): the first search starts after a short copy, and each part lands
+  // before the search stream reaches it.  A part costs about a millisecond of
+  // latency (its orientation and sort wait for the search before it) whatever
+  // its size: 12.5 to 12.9 ms for 1,024 graphs of 65 M arcs against 15.1 with
+  // six parts, 13.4 to 14.0 with four and 12.8 to 13.0 with two (10 and 54).
+  // Otherwise they are six equal ones.
   const bool pipelined = !o.log_roots && !o.warp_log && !o.count_ops &&
                          (o.sched == MCE_SCHED_PLAIN || o.sched == MCE_SCHED_DEGREE);
-  static const int64_t kGeo[MAX_PARTS] = {2, 6, 13, 24, 40, 64};  // cumulative 64ths
-  int k = m >= BATCH_PART_MIN_ARCS ? MAX_PARTS : 1;
+  static const int64_t kGeo[] = {6, 22, 64};  // cumulative 64ths
+  int k = m < BATCH_PART_MIN_ARCS ? 1 : pipelined ? 3 : MAX_PARTS;
   if (k > G) k = G;
   BatchParts P;
   P.k = 0;
   P.g[0] = 0;
   for (int p = 1; p < k; ++p) {
     int64_t gp = P.g[P.k];
-    const int64_t want = pipelined && k == MAX_PARTS ? m * kGeo[p - 1] / 64 : m * p / k;
+    const int64_t want = pipelined && k == 3 ? m * kGeo[p - 1] / 64 : m * p / k;
     while (gp < G && ao[gp] < want) ++gp;
     if (gp > P.g[P.k] && gp < G) P.g[++P.k] = gp;
   }
