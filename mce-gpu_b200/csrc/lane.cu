@@ -20,8 +20,10 @@
 // warp engine, which can share them; so do the roots with too many earlier
 // neighbours, whole.
 //
-// What bounds it: the divergence of 32 trees, in instructions; a lane's last
-// long tree at the end of a launch (hence LANE_DRAIN).  On the 2.86 M roots of
+// What bounds it: the latency of loading the next roots' rows (20 warps stalled
+// on loads per issue, 34 % of issue slots, on 512 graphs), then the divergence
+// of 32 trees (11 lanes active per instruction) and a lane's last long tree at
+// the end of a launch (hence LANE_DRAIN).  On the 2.86 M roots of
 // 1,024 Chung-Lu graphs the launch of up to 16 later neighbours takes 0.79 ms,
 // that of up to 32 (and 64 earlier ones) 0.50 ms and the warp engine's rest
 // 1.15 ms; the warp engine alone took 3.98 ms for all of them.
