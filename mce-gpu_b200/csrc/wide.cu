@@ -81,6 +81,15 @@ struct WSmem {
   u64 stk[WIDE_FRAMES][5 * W + 1];  // P, X, branches, settled leaves, chosen; list start and length
 };
 
+// A task of this engine: the root, then P, X and the chosen set, W words each.
+// Its size does not depend on the graph's widest root (bk_mem_kernel's does),
+// so that a lane of the taker holds one word.
+template <int W>
+constexpr uint32_t wide_task_words() {
+  static_assert(1 + 3 * W <= 32, "one word per lane");
+  return 1 + 3 * W;
+}
+
 // Slab of a warp, in words: the frames past the shared ones, then the lists
 // of earlier-neighbour rows (xcap rows).
 template <int W>
@@ -300,14 +309,14 @@ __device__ void w_tree(const BKArgs &a, WSmem<W> &sm, u64 *slab, const WRoot &rt
         recheck = 32;
       }
       if (want) {
-        const int WM = (a.dcap + 63) >> 6;
         if (q_push(a.q, [&](uint32_t k2) -> u64 {
-              if (k2 == 0) return (u64)(uint32_t)rt.r;
-              const int part = (int)(k2 - 1) / WM, w = (int)(k2 - 1) % WM;
-              u64 x = 0;
+              u64 x = (u64)(uint32_t)rt.r;
 #pragma unroll
-              for (int j = 0; j < W; ++j)
-                if (j == w) x = part == 0 ? Pc.w[j] : part == 1 ? Xc.w[j] : part == 2 ? Sc.w[j] : 0ull;
+              for (int j = 0; j < W; ++j) {
+                if ((int)k2 == 1 + j) x = Pc.w[j];
+                if ((int)k2 == 1 + W + j) x = Xc.w[j];
+                if ((int)k2 == 1 + 2 * W + j) x = Sc.w[j];
+              }
               return x;
             }))
           continue;
@@ -419,15 +428,22 @@ __device__ void w_tree(const BKArgs &a, WSmem<W> &sm, u64 *slab, const WRoot &rt
 }
 
 // The root's rows into shared memory; its earlier rows stay where they are.
+// False, with a status bit, for a root that is not this engine's: wider than
+// its sets, without rows, or with more earlier neighbours than the lists hold.
 template <int W>
-__device__ __forceinline__ void w_load(const BKArgs &a, WSmem<W> &sm, int32_t r, WRoot &rt) {
+__device__ __forceinline__ bool w_load(const BKArgs &a, WSmem<W> &sm, int32_t r, WRoot &rt) {
   const int lane = (int)lane_id();
   const int32_t ub = a.rp[r], sb = a.split[r];
-  rt.r = r;
-  rt.d = a.rp[r + 1] - sb;
-  rt.u = sb - ub;
-  rt.Wr = (rt.d + 63) >> 6;
+  const int d = a.rp[r + 1] - sb, u = sb - ub;
   const u64 *rows = a.wptr[r];
+  if (d > 64 * W || !rows || u > a.xcap) {
+    if (lane == 0) atomicOr(a.err, d > 64 * W || !rows ? MCE_ERR_DEGREE : MCE_ERR_XROWS);
+    return false;
+  }
+  rt.r = r;
+  rt.d = d;
+  rt.u = u;
+  rt.Wr = (rt.d + 63) >> 6;
   rt.xr = rows + (size_t)rt.d * rt.Wr;
   __syncwarp();
   for (int i = lane; i < rt.d; i += 32) {
@@ -435,6 +451,7 @@ __device__ __forceinline__ void w_load(const BKArgs &a, WSmem<W> &sm, int32_t r,
     for (int j = 0; j < W; ++j) sm.rows[i][j] = j < rt.Wr ? rows[(size_t)i * rt.Wr + j] : 0ull;
   }
   __syncwarp();
+  return true;
 }
 
 // The roots of the wide class with more than d_lo and at most 64 W later
@@ -459,7 +476,7 @@ __global__ void __launch_bounds__(W_BLOCK, W == 2 ? 5 : 4) wide_kernel(BKArgs a,
     const int32_t r = a.roots[i];
     const int d = a.rp[r + 1] - a.split[r];
     if (d <= d_lo || d > 64 * W) continue;  // another launch's
-    w_load<W>(a, sm, r, rt);
+    if (!w_load<W>(a, sm, r, rt)) continue;
     WSet<W> P, none;
     none.clear();
 #pragma unroll
@@ -471,8 +488,7 @@ __global__ void __launch_bounds__(W_BLOCK, W == 2 ? 5 : 4) wide_kernel(BKArgs a,
   }
   if (share) {
     root_phase_done(a.q);
-    const int WM = (a.dcap + 63) >> 6;
-    u64 t = 0;  // lane k: word k of the task (at most 1 + 4 * 4 words)
+    u64 t = 0;  // lane k: word k of the task
     idle_phase(
         a, [&](uint32_t, u64 w) { t = w; },
         [&]() {
@@ -480,14 +496,11 @@ __global__ void __launch_bounds__(W_BLOCK, W == 2 ? 5 : 4) wide_kernel(BKArgs a,
           WSet<W> P, X, S;
 #pragma unroll
           for (int j = 0; j < W; ++j) {
-            const u64 p = __shfl_sync(MCE_FULL, t, (1 + j) & 31);
-            const u64 x = __shfl_sync(MCE_FULL, t, (1 + WM + j) & 31);
-            const u64 c = __shfl_sync(MCE_FULL, t, (1 + 2 * WM + j) & 31);
-            P.w[j] = j < WM ? p : 0ull;
-            X.w[j] = j < WM ? x : 0ull;
-            S.w[j] = j < WM ? c : 0ull;
+            P.w[j] = __shfl_sync(MCE_FULL, t, 1 + j);
+            X.w[j] = __shfl_sync(MCE_FULL, t, 1 + W + j);
+            S.w[j] = __shfl_sync(MCE_FULL, t, 1 + 2 * W + j);
           }
-          if (r != rt.r) w_load<W>(a, sm, r, rt);
+          if (r != rt.r && !w_load<W>(a, sm, r, rt)) return;
           u64 nd = 0, cnt = 0;
           w_tree<W, XP>(a, sm, slab, rt, P, X, S, h0, h1, nd, cnt);
           nodes += nd;
@@ -521,8 +534,14 @@ int wide_plan(int W, bool xp, int sms, int xcap, int *grid, size_t *slab_words) 
   return xp ? w_plan<4, true>(sms, grid) : w_plan<4, false>(sms, grid);
 }
 
-int wide_launch(int W, bool xp, const BKArgs &a, int d_lo, int fetch, int grid, cudaStream_t s,
+int wide_launch(int W, bool xp, const BKArgs &args, int d_lo, int fetch, int grid, cudaStream_t s,
                 int *launches) {
+  BKArgs a = args;
+  if (a.q.hdr) {  // the ring's slots are sized for the graph's widest root: at least as long
+    const uint32_t words = W == 2 ? wide_task_words<2>() : wide_task_words<4>();
+    if (a.q.words < words) return MCE_EINVAL;
+    a.q.words = words;
+  }
   const size_t smem = (W == 2 ? sizeof(WSmem<2>) : sizeof(WSmem<4>)) * (W_BLOCK / 32);
   if (W == 2 && xp)
     wide_kernel<2, true><<<grid, W_BLOCK, smem, s>>>(a, d_lo, fetch);

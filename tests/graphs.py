@@ -90,3 +90,26 @@ KNOWN = [
     ("petersen", petersen, 15, {2: 15}),
     ("empty50", lambda: empty(50), 0, {}),
 ]
+
+
+def core(clique, chain, missing, around, seed):
+    """A dense core with wide roots whose trees branch, deeply and with few
+    cliques: `clique` vertices adjacent to everything in the core, 2 `chain`
+    vertices of which a_i and b_j are not adjacent where i <= j (the search
+    descends a vertex of the chain at a time, a branch open at each level),
+    `missing` more pairs without an edge, and `around` vertices outside it,
+    each adjacent to three fifths of the core."""
+    rng = np.random.default_rng(seed)
+    n = clique + 2 * chain
+    adj = np.ones((n, n), bool)
+    for i in range(chain):
+        adj[i, chain + i:2 * chain] = False
+    rest = rng.choice(np.arange(2 * chain, n), 2 * missing, replace=False)
+    adj[rest[::2], rest[1::2]] = False
+    i, j = np.nonzero(np.triu(adj & adj.T, 1))
+    out = [(n + v, int(u)) for v in range(around) for u in rng.choice(n, 3 * n // 5, replace=False)]
+    perm = np.arange(n + around)
+    perm[2 * chain:] = 2 * chain + rng.permutation(n + around - 2 * chain)
+    src = np.concatenate([i, [a for a, _ in out]]).astype(np.int64)
+    dst = np.concatenate([j, [b for _, b in out]]).astype(np.int64)
+    return mce.from_edges(perm[src], perm[dst], n + around)
