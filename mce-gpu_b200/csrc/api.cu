@@ -1190,7 +1190,8 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
         for (const WideLaunch &l : wl) {
           a.slab_words = l.slab_words;
           a.d_lo = l.d_lo;
-          if (share && (r2 = queue_launch_init(a.q, s, &launches))) return r2;
+          // one ring for the class's launches: `pushed` adds up over them
+          if (share && (r2 = queue_launch_init(a.q, s, &launches, &l != &wl[0]))) return r2;
           if ((r2 = l.W ? wide_launch(l.W, a.x_pivot != 0, a, l.d_lo, l.fetch, l.grid, s, &launches)
                         : bk_launch(c, wbits, a, l.grid, l.block, 0, s, &launches)))
             return r2;

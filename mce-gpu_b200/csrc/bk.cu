@@ -24,6 +24,7 @@
 // Tie-breaking: the pivot with the lowest index among the best scores, so
 // per-root tree sizes are deterministic and independent of who walks them.
 #include <climits>
+#include <cstddef>
 #include <cstring>
 
 #include "common.cuh"
@@ -434,8 +435,8 @@ int bk_launch(int cls, int word_bits, const BKArgs &a, int grid, int block, int 
   return rc;
 }
 
-int queue_launch_init(const QueueView &q, cudaStream_t s, int *launches) {
-  MCE_CUDA(cudaMemsetAsync(q.hdr, 0, sizeof(QueueHdr), s));
+int queue_launch_init(const QueueView &q, cudaStream_t s, int *launches, bool keep_pushed) {
+  MCE_CUDA(cudaMemsetAsync(q.hdr, 0, keep_pushed ? offsetof(QueueHdr, pushed) : sizeof(QueueHdr), s));
   queue_init_kernel<<<(q.cap + 255) / 256, 256, 0, s>>>(q);
   MCE_CUDA(cudaGetLastError());
   if (launches) *launches += 1;

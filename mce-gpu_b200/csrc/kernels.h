@@ -219,7 +219,7 @@ int wide_launch(int W, bool xp, const BKArgs &a, int d_lo, int fetch, int grid, 
 int bk_warps_for_class(int cls, int sms, int wide_blocks, int *warps, int *block, int *smem);
 size_t bk_slab_words(int cls, int dcap, int xcap, int rxcap = REG_XCAP);
 uint32_t bk_task_words(int cls, int dcap);
-int queue_launch_init(const QueueView &q, cudaStream_t s, int *launches);
+int queue_launch_init(const QueueView &q, cudaStream_t s, int *launches, bool keep_pushed = false);
 
 // ---- cost model -----------------------------------------------------------------
 constexpr int MLP_IN = 8, MLP_HIDDEN = 64;

@@ -32,7 +32,7 @@ struct QueueHdr {  // one word per 128-byte line
   uint32_t pad1[31];
   uint32_t work;   // see above
   uint32_t pad2[31];
-  uint32_t pushed; // statistics
+  uint32_t pushed; // tasks pushed, over all launches of a search on this ring (statistics)
 };
 
 struct QueueView {

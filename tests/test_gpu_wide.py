@@ -38,6 +38,15 @@ def test_roots_match_oracle(name, kw):
         assert dg.count(level=mce.LEVEL_L2, **kw).total == tot
 
 
+@pytest.mark.parametrize("name,threshold", [("cores up to 240", 129), ("a core of 680", 257)])
+def test_donations_of_every_wide_launch(name, threshold):
+    """Subtrees of so many candidates come from the first launches only."""
+    with mce.Graph.from_host(together(GRAPHS[name]())) as dg:
+        for graph in (0, 1):
+            r = dg.count(donate_after=1, donate_threshold=threshold, cuda_graph=graph)
+            assert r.stats["donations"] > 0
+
+
 @pytest.mark.parametrize("kw", [{}, SHARED, {"x_pivot": 1, "donate_after": 1}], ids=str)
 def test_batches_match_oracle(kw):
     gs = GRAPHS["beside a clique of 1000"]() + CORES
