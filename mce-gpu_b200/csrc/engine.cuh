@@ -135,7 +135,7 @@ __device__ void idle_phase(const BKArgs &a, Put put, Run run) {
         } else if ((polls++ & 3u) == 0) {
           const uint32_t work = ld_volatile(&q.hdr->work);
           if (work == 0) {
-            if (q_leave(q, pos)) state = 2;
+            state = 2;  // every root is walked and no task is left: none will come
           } else {  // pushes move tail, ends of tasks and root phases move work
             const uint32_t now_at = ld_volatile(&q.hdr->tail) * 2654435761u + work;
             const uint64_t now = globaltimer_ns();
@@ -144,7 +144,6 @@ __device__ void idle_phase(const BKArgs &a, Put put, Run run) {
               t_last = now;
             } else if (now - t_last > a.wait_limit_ns) {
               atomicOr(a.err, MCE_ERR_WAIT_TIMEOUT);  // no progress anywhere: give up
-              q_leave(q, pos);
               state = 2;
             }
           }
@@ -1141,7 +1140,7 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
       if (want) {
         const u64 w0 = (u64)(uint32_t)rt.r, w1 = (u64)Pc, w2 = (u64)Xc, w3 = (u64)Sc,
                   w4 = L2 ? (u64)XO : 0ull;
-        if (q_push(a.q, [&](uint32_t k2) {
+        if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) {
               return k2 == 0 ? w0 : k2 == 1 ? w1 : k2 == 2 ? w2 : k2 == 3 ? w3 : w4;
             })) {
           if (EV && lane == 0) warp_record(a)[2] += 1;  // opts.warp_log
@@ -1769,7 +1768,7 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
       MCE_BD(BD_QUEUE);
       const int WM = (a.dcap + 63) >> 6;
       const u64 *Cp = C, *Cx = C + Wr, *Cs = C + 3 * Wr;
-      if (q_push(a.q, [&](uint32_t k2) -> u64 {
+      if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
             if (k2 == 0) return (u64)(uint32_t)rt.r;
             const uint32_t part = (k2 - 1) / WM, w = (k2 - 1) % WM;
             if ((int)w >= Wr) return 0ull;

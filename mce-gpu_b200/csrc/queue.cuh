@@ -18,7 +18,7 @@
 // donors agreeing on the ring's tail by compare-and-swap the device made one
 // push per 0.9 us, and the time of the search of an R-MAT graph of scale 13
 // was its number of pushes.  An idle warp's poll is bounded by a no-progress
-// time limit, a donor's wait for its slot by a count.
+// time limit, a donor's wait for its slot by the same time.
 #pragma once
 
 #include "common.cuh"
@@ -45,35 +45,42 @@ struct QueueView {
 
 __global__ void queue_init_kernel(QueueView q);
 
-// A ring slot at position pos (modulo cap): seq = pos when empty, pos + 2
-// while a donor writes its task, pos + 1 with the task there, pos + cap once
-// the task was taken - or its ticket given up by a warp that left.
+// A ring slot at position pos (modulo cap): seq = pos when empty, pos + 1 with
+// the task there, pos + cap once the task was taken.
 //
-// Claim a slot and publish `words` task words held by the warp (lane k holds
-// words k, k+32, ...; supplied by `get(k)`).  Returns false if full.
+// Claim a position and publish `words` task words held by the warp (lane k
+// holds words k, k+32, ...; supplied by `get(k)`).  Returns false if the ring
+// is full: a position is only claimed while positions run less than a lap,
+// minus one per warp of the launch, ahead of tickets.  Even with every warp
+// past that test at once the position stays less than a lap ahead, so the
+// ticket of its slot's last task is drawn and the wait for the slot is one for
+// a running warp to copy a task out.  That wait is bounded by limit_ns: when it
+// runs out the search ends with MCE_ERR_WAIT_TIMEOUT.
 template <typename Get>
-__device__ __forceinline__ bool q_push(const QueueView &q, Get get) {
+__device__ __forceinline__ bool q_push(const QueueView &q, uint32_t *err, uint64_t limit_ns,
+                                       Get get) {
   const uint32_t lane = lane_id();
   uint32_t pos = 0;
   int ok = 0;
   if (lane == 0) {
-    for (int tries = 0; tries < 64 && !ok; ++tries) {
+    const int32_t room = (int32_t)q.cap - (int32_t)(gridDim.x * (blockDim.x >> 5));
+    if ((int32_t)(ld_volatile(&q.hdr->tail) - ld_volatile(&q.hdr->head)) < room) {
       pos = atomicAdd(&q.hdr->tail, 1u);
-      uint32_t *s = &q.seq[pos & (q.cap - 1)];
-      uint32_t seen = atomicCAS(s, pos, pos + 2);
-      // a task of the ring's last lap whose taker is still reading it (the ring
-      // is twice as long as there are warps)
-      for (int spin = 0; seen != pos && seen != pos + q.cap && spin < (1 << 20); ++spin) {
-        __nanosleep(64);
-        seen = atomicCAS(s, pos, pos + 2);
+      const uint32_t *s = &q.seq[pos & (q.cap - 1)];
+      ok = ld_acquire(s) == pos;
+      if (!ok) {
+        const uint64_t t0 = globaltimer_ns();
+        do {
+          __nanosleep(64);
+          ok = ld_acquire(s) == pos;
+        } while (!ok && globaltimer_ns() - t0 <= limit_ns);
       }
-      if (seen == pos) {
+      if (ok) {
         atomicAdd(&q.hdr->work, 1u);  // counted before anyone can take it
         atomicAdd(&q.hdr->pushed, 1u);
-        ok = 1;
-      } else if (seen != pos + q.cap) {
-        break;  // the wait ran out: keep the subtree
-      }  // else: a ticket that was given up, try the next position
+      } else {
+        atomicOr(err, MCE_ERR_WAIT_TIMEOUT);
+      }
     }
   }
   ok = __shfl_sync(MCE_FULL, ok, 0);
@@ -93,11 +100,6 @@ __device__ __forceinline__ bool q_push(const QueueView &q, Get get) {
 // Whether the task of ticket `pos` is there (lane 0's answer).
 __device__ __forceinline__ bool q_ready(const QueueView &q, uint32_t pos) {
   return ld_acquire(&q.seq[pos & (q.cap - 1)]) == pos + 1;
-}
-
-// Give ticket `pos` up (lane 0): false if a donor has its slot already.
-__device__ __forceinline__ bool q_leave(const QueueView &q, uint32_t pos) {
-  return atomicCAS(&q.seq[pos & (q.cap - 1)], pos, pos + q.cap) == pos;
 }
 
 // Take the task of ticket `pos` (q_ready on lane 0 said so): put(k, word)

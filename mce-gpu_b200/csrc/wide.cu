@@ -309,7 +309,7 @@ __device__ void w_tree(const BKArgs &a, WSmem<W> &sm, u64 *slab, const WRoot &rt
         recheck = 32;
       }
       if (want) {
-        if (q_push(a.q, [&](uint32_t k2) -> u64 {
+        if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
               u64 x = (u64)(uint32_t)rt.r;
 #pragma unroll
               for (int j = 0; j < W; ++j) {
