@@ -171,10 +171,12 @@ __device__ __forceinline__ int32_t lower_bound_g(const int32_t *__restrict__ a, 
 }
 
 // The row of v's earlier neighbour x (its place in v's earlier list found by
-// binary search), at most 64 bits wide.
+// binary search), at most 64 bits wide.  In a CSR that is not symmetric x may
+// not be there: its place past the list has no row.
 __device__ __forceinline__ void put_row(const EncArgs &a, int32_t x, int32_t v, int32_t rv,
                                         int dv, int uv, uint32_t lo, uint32_t hi) {
   const int32_t pos = lower_bound_g(a.cs + rv, uv, x);
+  if (pos >= uv) return;
   if (dv <= 32 && uv <= REG_XCAP_MAX) {
     a.enc[rv + pos] = lo;
   } else {
@@ -219,6 +221,7 @@ __device__ __forceinline__ void long_item(const EncArgs &a, int32_t x, int32_t v
   unsigned long long *p = a.wptr[v];
   if (!p) return;
   const int32_t pos = lower_bound_g(a.cs + rv, sv - rv, x);  // the same for every lane
+  if (pos >= sv - rv) return;  // as in put_row
   uint32_t *dst = reinterpret_cast<uint32_t *>(p + ((size_t)dv + pos) * W);
   if (lane < 2 * W) dst[lane] = w0;
   if (lane + 32 < 2 * W) dst[lane + 32] = w1;

@@ -34,7 +34,16 @@ using std::min;
 typedef void *cudaStream_t;
 typedef void *cudaEvent_t;
 enum cudaError_t { cudaSuccess = 0 };
-enum { cudaFuncAttributeMaxDynamicSharedMemorySize, cudaDevAttrMultiProcessorCount, cudaDevAttrCooperativeLaunch };
+enum {
+  cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaDevAttrMultiProcessorCount,
+  cudaDevAttrCooperativeLaunch,
+  cudaMemcpyDeviceToHost
+};
+struct dim3 {
+  unsigned x;
+  dim3(unsigned n) : x(n) {}
+};
 struct int2 {
   int x, y;
 };
@@ -263,6 +272,25 @@ inline cudaError_t cudaGetLastError() { return cudaSuccess; }
 inline cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) {
   memset(p, v, n);
   return cudaSuccess;
+}
+inline cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, int, cudaStream_t) {
+  memcpy(to, from, n);
+  return cudaSuccess;
+}
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+inline cudaError_t cudaGetDevice(int *d) {
+  *d = 0;
+  return cudaSuccess;
+}
+inline cudaError_t cudaDeviceGetAttribute(int *v, int, int) {
+  *v = 1;
+  return cudaSuccess;
+}
+inline cudaError_t cudaLaunchCooperativeKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) {
+  fprintf(stderr, "no grid barriers here: a block runs at a time\n");
+  exit(5);
 }
 template <typename F>
 cudaError_t cudaFuncSetAttribute(F, int, int) {
