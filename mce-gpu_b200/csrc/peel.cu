@@ -623,14 +623,16 @@ __device__ void peel_graph_smem(const int32_t *__restrict__ rp, const int32_t *_
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&sh.cnt[ph], (uint32_t)(__popc(m0) + __popc(m1)));
         base = __shfl_sync(MCE_FULL, base, 0) + (uint32_t)head;
-        if (t0) order[base + __popc(m0 & lt)] = (uint16_t)(2 * k);
-        if (t1) order[base + __popc(m0) + __popc(m1 & lt)] = (uint16_t)(2 * k + 1);
+        // below n, unless repeated or one-sided arcs wore a removed vertex's mark down
+        const uint32_t p0 = base + __popc(m0 & lt), p1 = base + __popc(m0) + __popc(m1 & lt);
+        if (t0 && p0 < (uint32_t)n) order[p0] = (uint16_t)(2 * k);
+        if (t1 && p1 < (uint32_t)n) order[p1] = (uint16_t)(2 * k + 1);
       }
     }
     mn = __reduce_min_sync(MCE_FULL, mn);
     if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(&sh.mn[ph], mn);
     __syncthreads();
-    int cnt = (int)sh.cnt[ph];
+    int cnt = min((int)sh.cnt[ph], n - head);
     const uint32_t lowest = sh.mn[ph];
     next_phase();
     if (cnt == 0) {  // no vertex at this level: go to the lowest remaining degree

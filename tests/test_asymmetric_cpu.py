@@ -5,6 +5,8 @@ import numpy as np
 import pytest
 
 import emulate
+import mce_b200 as mce
+import oracle
 
 
 def directed(n, rows):
@@ -33,8 +35,35 @@ def forward(n, p, seed):
     return directed(n, [np.nonzero(r)[0] for r in a[:-1]] + [[0]])
 
 
+def repeated(targets=6, pointing=40, rest=30, arcs=32000):
+    """Arcs repeated so often that the targets, whose rows are short, are pointed
+    at by more arcs than a 16-bit degree holds beside its mark, before a rest of
+    vertices of higher degree is peeled."""
+    n = targets + pointing + rest
+    return directed(n, [[targets]] * targets +
+                    [np.repeat(np.arange(targets), arcs // pointing)] * pointing +
+                    [np.repeat([v for v in range(n - rest, n) if v != n - rest + b], 200)
+                     for b in range(rest)])
+
+
 GRAPHS = {"pointed at": pointed_at(200, list(range(40, 80))), "thinned": thinned(300, 0.3, 0.6, 1),
           "thinned, dense": thinned(260, 0.9, 0.9, 2), "forward": forward(280, 0.5, 3)}
+
+
+@pytest.mark.parametrize("name", list(GRAPHS) + ["repeated"])
+def test_peel_stays_in_its_shared_memory(name):
+    rp, col = repeated() if name == "repeated" else GRAPHS[name]
+    rc, _, err = emulate.run("peel", arrays=(rp, col), timeout=60)
+    assert rc == 0, err
+
+
+def test_peel_of_a_symmetric_graph():
+    g = mce.gen_er(301, 0.1, 4, 3, 10, 30)
+    rc, out, err = emulate.run("peel", arrays=(g.row_ptr[:g.n + 1], g.col), timeout=60)
+    assert rc == 0, err
+    prio, core, _ = oracle.peel(g)
+    x = np.frombuffer(out, np.uint32)
+    assert np.array_equal(x[:g.n], prio) and np.array_equal(x[g.n:], core)
 
 
 @pytest.mark.parametrize("name", GRAPHS)
