@@ -15,6 +15,7 @@
 #include "../host/host.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "scratch.h"
 
 namespace mce {
 
@@ -489,27 +490,52 @@ int run_parts(mce_graph *g, cudaStream_t s, int *launches, const BatchCtx *bc, i
   return MCE_OK;
 }
 
-// The rows of every root of a summary (part i - 1 of a batch, or i = 0: the
-// whole graph) before its search.  The wide roots' rows are bounded by
-// WIDE_BYTES and by what the device has left: the search encodes the rest.
-constexpr uint64_t WIDE_BYTES = 32ull << 30;
 constexpr uint32_t ROWS_MIN_ROOTS = 16384, ROWS_MAX_EARLIER = 256;
 constexpr uint32_t SHARE_MIN_LATER = 16;
 
+// Words of wide roots' rows that region i may have (scratch.h) for a call that
+// allocates `needed` bytes more.
+int rows_grant(mce_graph *g, int i, uint64_t words, uint64_t needed, uint64_t *granted) {
+  *granted = words;
+  if (8 * words <= WIDE_UNASKED) return MCE_OK;
+  uint64_t others = 0;
+  for (int j = 0; j < 1 + MAX_PARTS; ++j)
+    if (j != i) others += 8 * g->wide_cap[j];
+  size_t free_now = 0, all = 0;
+  MCE_CUDA(cudaMemGetInfo(&free_now, &all));
+  *granted = wide_grant(8 * words, 8 * g->wide_cap[i], others, free_now, needed) / 8;
+  return MCE_OK;
+}
+
+// Gives every region of rows back (the search then encodes the wide roots
+// itself); false if there was none.
+bool drop_rows(mce_graph *g, cudaStream_t s) {
+  (void)cudaGetLastError();  // the allocation that failed
+  bool any = false;
+  for (int j = 0; j < 1 + MAX_PARTS; ++j) any = any || g->wide[j];
+  if (!any || cudaStreamSynchronize(s) != cudaSuccess) return false;
+  for (int j = 0; j < 1 + MAX_PARTS; ++j) {
+    dfree(g->wide[j]);
+    g->wide_cap[j] = 0;
+  }
+  g->wide_all = false;
+  return cudaMemsetAsync(g->wptr, 0, sizeof(*g->wptr) * ((size_t)g->n + 1), s) == cudaSuccess;
+}
+
+// The rows of every root of a summary (part i - 1 of a batch, or i = 0: the
+// whole graph) before its search.  The wide roots' rows are optional: their
+// region grows to `granted` words (rows_grant) after the search's other buffers
+// are there, and the search encodes the roots past it.
 int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const ShapeInfo *shape_dev,
             int i, const int32_t *wide_list, const unsigned long long *wide_off, int64_t arc0,
-            int64_t arc1, int64_t v0, int64_t v1, cudaStream_t s, int *launches) {
-  const uint64_t want = std::min<uint64_t>(sh.wide_words, WIDE_BYTES / 8);
-  if (want > g->wide_cap[i]) {
+            int64_t arc1, int64_t v0, int64_t v1, uint64_t granted, cudaStream_t s, int *launches) {
+  if (granted > g->wide_cap[i]) {
     dfree(g->wide[i]);
-    g->wide_cap[i] = 0;
-    for (uint64_t w = want; w > 0; w /= 2) {
-      if (cudaMalloc((void **)&g->wide[i], sizeof(unsigned long long) * w) == cudaSuccess) {
-        g->wide_cap[i] = w;
-        break;
-      }
+    g->wide_cap[i] = granted;
+    if (cudaMalloc((void **)&g->wide[i], 8 * granted) != cudaSuccess) {
       g->wide[i] = nullptr;
-      (void)cudaGetLastError();  // too large for what is left: try half
+      g->wide_cap[i] = 0;
+      (void)cudaGetLastError();  // taken by another process meanwhile: no rows
     }
   }
   if (sh.wide_words > g->wide_cap[i]) g->wide_all = false;
@@ -524,9 +550,9 @@ int run_enc(mce_graph *g, const ShapeInfo &sh, const int32_t *roots, const Shape
   ea.wptr = g->wptr;
   ea.nx = g->nx;
   ea.next = g->enc_next + i;
-  return enc_launch(ea, wide_list, sh.wide_cnt, wide_off, g->wide[i],
-                    std::min<uint64_t>(want, g->wide_cap[i]), sh.cls_cnt[CLS_R32], sh.max_dplus,
-                    arc0, arc1, v0, v1, g->sms, s, launches);
+  const uint64_t words = std::min<uint64_t>(sh.wide_words, g->wide_cap[i]);
+  return enc_launch(ea, wide_list, sh.wide_cnt, wide_off, g->wide[i], words, sh.cls_cnt[CLS_R32],
+                    sh.max_dplus, arc0, arc1, v0, v1, g->sms, s, launches);
 }
 
 // The launches of the wide class, widest roots first: bk_mem_kernel (W = 0)
@@ -969,15 +995,21 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   if ((rc = read_shape(g, s))) return rc;
   const ShapeInfo &sh = g->shape_h;
   if (sh.cls_cnt[CLS_BIG]) return MCE_ELIMIT;
-  g->wide_all = true;
   // A few thousand narrow roots without hubs are encoded by the search's own
   // warps: building their rows first would only add launches (ER n = 200 254
   // against 236 us, n = 10,000 461 against 441 us a call).
   const bool rows = sh.wide_cnt > 0 || sh.cls_cnt[CLS_R32] >= ROWS_MIN_ROOTS ||
                     sh.max_dminus_reg > ROWS_MAX_EARLIER;
-  if (rows && (rc = run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0,
-                            g->n, s, &launches)))
-    return rc;
+  // Rows that fit what the handle holds are built at once, beside the host's
+  // planning; otherwise after the buffers that the search cannot do without.
+  const bool grow = rows && sh.wide_words > g->wide_cap[0];
+  uint64_t granted = g->wide_cap[0];
+  auto build_rows = [&]() {
+    return run_enc(g, sh, g->roots, g->shape, 0, g->wide_list, g->wide_off, 0, g->m, 0, g->n,
+                   granted, s, &launches);
+  };
+  g->wide_all = true;
+  if (rows && !grow && (rc = build_rows())) return rc;
   // search scratch
   // Trees over at most 16 later neighbours have a few hundred nodes: nothing
   // to share, and no idle warps to launch for it.
@@ -987,7 +1019,6 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   const int xcap = (int)(sh.max_dminus_mem > 0 ? sh.max_dminus_mem : 1);
   int rxcap = REG_XCAP;  // a power of two covering the register classes' earlier degrees
   while (rxcap < (int)sh.max_dminus_reg && rxcap < REG_XCAP_MAX) rxcap <<= 1;
-  size_t slab_need = 0;
   // per bucket (engine class): warps per root, donation threshold and gate
   int parts[NCLS] = {1, 1, 1, 1, 1}, dmin[NCLS] = {0}, dafter[NCLS] = {0};
   for (int c = CLS_R32; c <= CLS_MEM; ++c) {
@@ -999,50 +1030,88 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     const int af = o.bucket_donate_after[c] ? o.bucket_donate_after[c] : o.donate_after;
     dafter[c] = af > 0 ? af : (int)DEFAULT_DONATE_AFTER;
   }
+  const bool lanes = use_lanes(o, sh.cls_cnt[CLS_R32], parts[CLS_R32], lc != nullptr);
   std::vector<WideLaunch> wl;
-  if (sh.cls_cnt[CLS_MEM]) {
-    if ((rc = plan_wide(g, o, parts[CLS_MEM], lc != nullptr, dcap, xcap, &wl))) return rc;
-    block[CLS_MEM] = MEM_THREADS;
-    for (WideLaunch &l : wl) {
-      if (!share) {  // never more warps than units of work
-        const int64_t units = (int64_t)sh.cls_cnt[CLS_MEM] * parts[CLS_MEM];
-        l.grid = (int)std::min<int64_t>(l.grid, (units + 3) / 4);
+  size_t slab_need = 0;
+  // the launches, as g->wide_all allows
+  auto plan = [&]() -> int {
+    slab_need = 0;
+    grid[CLS_MEM] = 0;
+    if (sh.cls_cnt[CLS_MEM]) {
+      int r = plan_wide(g, o, parts[CLS_MEM], lc != nullptr, dcap, xcap, &wl);
+      if (r) return r;
+      block[CLS_MEM] = MEM_THREADS;
+      for (WideLaunch &l : wl) {
+        if (!share) {  // never more warps than units of work
+          const int64_t units = (int64_t)sh.cls_cnt[CLS_MEM] * parts[CLS_MEM];
+          l.grid = (int)std::min<int64_t>(l.grid, (units + 3) / 4);
+        }
+        grid[CLS_MEM] = std::max(grid[CLS_MEM], l.grid);
+        slab_need = std::max(slab_need, (size_t)l.grid * 4 * l.slab_words * 8);
       }
-      grid[CLS_MEM] = std::max(grid[CLS_MEM], l.grid);
-      slab_need = std::max(slab_need, (size_t)l.grid * 4 * l.slab_words * 8);
     }
-  }
-  for (int c = CLS_R32; c <= CLS_R64; ++c) {
-    if (!sh.cls_cnt[c]) continue;
-    int warps = 0;
-    if ((rc = bk_warps_for_class(c, g->sms, o.wide_blocks, &warps, &block[c], &smem[c]))) return rc;
-    // never more warps than units of work (a root's parts; rounded up to
-    // whole blocks); with task sharing keep at least a full wave so idle
-    // warps can take subtrees
-    const int wpb = block[c] / 32;
-    int64_t want = (int64_t)sh.cls_cnt[c] * parts[c];
-    if (share) want = want > warps ? want : warps;
-    if (want < warps) warps = (int)((want + wpb - 1) / wpb) * wpb;
-    grid[c] = warps / wpb;
-    const size_t need = (size_t)warps * bk_slab_words(c, dcap, xcap, rxcap) * 8;
-    if (need > slab_need) slab_need = need;
-  }
-  if ((rc = ensure_slab(g, slab_need))) return rc;
-  if (o.log_roots && !g->root_nodes) {
-    if ((rc = dalloc(&g->root_nodes, (size_t)g->cap_n + 1))) return rc;
-    if ((rc = dalloc(&g->root_count, (size_t)g->cap_n + 1))) return rc;
-  }
+    for (int c = CLS_R32; c <= CLS_R64; ++c) {
+      if (!sh.cls_cnt[c]) continue;
+      int warps = 0;
+      int r = bk_warps_for_class(c, g->sms, o.wide_blocks, &warps, &block[c], &smem[c]);
+      if (r) return r;
+      // never more warps than units of work (a root's parts; rounded up to
+      // whole blocks); with task sharing keep at least a full wave so idle
+      // warps can take subtrees
+      const int wpb = block[c] / 32;
+      int64_t want = (int64_t)sh.cls_cnt[c] * parts[c];
+      if (share) want = want > warps ? want : warps;
+      if (want < warps) warps = (int)((want + wpb - 1) / wpb) * wpb;
+      grid[c] = warps / wpb;
+      const size_t need = (size_t)warps * bk_slab_words(c, dcap, xcap, rxcap) * 8;
+      if (need > slab_need) slab_need = need;
+    }
+    return MCE_OK;
+  };
   const bool log_ops = o.log_roots && o.count_ops;
-  if (log_ops && !g->root_ops && (rc = dalloc(&g->root_ops, (size_t)g->cap_n + 1))) return rc;
   int64_t wlog_base[NCLS] = {0}, wlog_total = 0;
-  for (int c : {CLS_MEM, CLS_R64, CLS_R32}) {  // the launch order below
-    wlog_base[c] = wlog_total;
-    if (grid[c]) wlog_total += (int64_t)grid[c] * (block[c] / 32);
+  QueueView qv[NCLS];
+  // plans the launches and allocates what they need
+  auto reserve = [&]() -> int {
+    int r;
+    if ((r = plan()) || (r = ensure_slab(g, slab_need))) return r;
+    for (int c = CLS_R32; c <= CLS_MEM; ++c)
+      if (share && grid[c] && (r = ensure_queue(g, c, bk_task_words(c, dcap), &qv[c]))) return r;
+    if (lanes && !g->lane_resume &&
+        (r = dalloc(&g->lane_resume, (size_t)RESUME_CAP * RESUME_WORDS)))
+      return r;
+    if (o.log_roots && ((!g->root_nodes && (r = dalloc(&g->root_nodes, (size_t)g->cap_n + 1))) ||
+                        (!g->root_count && (r = dalloc(&g->root_count, (size_t)g->cap_n + 1)))))
+      return r;
+    if (log_ops && !g->root_ops && (r = dalloc(&g->root_ops, (size_t)g->cap_n + 1))) return r;
+    wlog_total = 0;
+    for (int c : {CLS_MEM, CLS_R64, CLS_R32}) {  // the launch order below
+      wlog_base[c] = wlog_total;
+      if (grid[c]) wlog_total += (int64_t)grid[c] * (block[c] / 32);
+    }
+    if (o.warp_log && wlog_total > g->wlog_cap) {
+      dfree(g->wlog);
+      g->wlog_cap = 0;
+      if ((r = dalloc(&g->wlog, WLOG_WORDS * (size_t)wlog_total))) return r;
+      g->wlog_cap = wlog_total;
+    }
+    return MCE_OK;
+  };
+  auto drop = [&]() {
+    granted = 0;
+    return drop_rows(g, s);
+  };
+  if (grow) {  // do all of them fit beside the slab of launches for roots with rows?
+    if ((rc = plan())) return rc;
+    const uint64_t needed = slab_need > g->slab_bytes ? slab_need - g->slab_bytes : 0;
+    if ((rc = rows_grant(g, 0, sh.wide_words, needed, &granted))) return rc;
+    g->wide_all = granted >= sh.wide_words;
   }
-  if (o.warp_log && wlog_total > g->wlog_cap) {
-    dfree(g->wlog);
-    if ((rc = dalloc(&g->wlog, WLOG_WORDS * (size_t)wlog_total))) return rc;
-    g->wlog_cap = wlog_total;
+  if ((rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
+  if (grow) {
+    const bool planned = g->wide_all;
+    if ((rc = build_rows())) return rc;
+    if (g->wide_all != planned && (rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
   }
   g->wlog_count = o.warp_log ? wlog_total : 0;
   BKArgs a;
@@ -1085,13 +1154,6 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     a.list_cap = lc->cap;
   }
   const int wbits = o.bitmap_width == 64 ? 64 : 32;
-  const bool lanes = use_lanes(o, sh.cls_cnt[CLS_R32], parts[CLS_R32], lc != nullptr);
-  if (lanes && !g->lane_resume &&
-      (rc = dalloc(&g->lane_resume, (size_t)RESUME_CAP * RESUME_WORDS)))
-    return rc;
-  QueueView qv[NCLS];
-  for (int c = CLS_R32; c <= CLS_MEM; ++c)
-    if (share && grid[c] && (rc = ensure_queue(g, c, bk_task_words(c, dcap), &qv[c]))) return rc;
   // Everything from here to the end of the search is a fixed sequence of
   // memsets and launches whose arguments depend only on `key`: with
   // opts.cuda_graph it is captured once and replayed.
@@ -1434,6 +1496,15 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
   };
   std::vector<Seg> defer[2];  // by class: R64, MEM (offsets into g->roots)
   uint32_t mx_dplus = 0, mx_dm_mem = 0, mx_dm_reg = 0, mx_deg = 0;
+  auto grow_slab = [&](size_t need) -> int {
+    if (need <= g->slab_bytes) return MCE_OK;
+    if (g->slab) retired.push_back(g->slab);  // earlier searches of the call keep the old one
+    g->slab = nullptr;
+    g->slab_bytes = 0;
+    MCE_CUDA(cudaMalloc((void **)&g->slab, need));
+    g->slab_bytes = need;
+    return MCE_OK;
+  };
   // grid, slab and queue of one class launch; returns MCE_OK or an error
   auto plan = [&](int c, int64_t roots, int dcap, int xcap, int rxcap, int *grid, int *block,
                   int *smem, int *parts_c, int *dmin_c, int *dafter_c, QueueView *qv) -> int {
@@ -1451,14 +1522,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     if (share_q) want = want > warps ? want : warps;
     if (want < warps) warps = (int)((want + wpb - 1) / wpb) * wpb;
     *grid = warps / wpb;
-    const size_t need = (size_t)warps * bk_slab_words(c, dcap, xcap, rxcap) * 8;
-    if (need > g->slab_bytes) {  // earlier searches of the call keep the old slab
-      if (g->slab) retired.push_back(g->slab);
-      g->slab = nullptr;
-      g->slab_bytes = 0;
-      MCE_CUDA(cudaMalloc((void **)&g->slab, need));
-      g->slab_bytes = need;
-    }
+    if ((r = grow_slab((size_t)warps * bk_slab_words(c, dcap, xcap, rxcap) * 8))) return r;
     if (share_q) {
       const uint32_t words = bk_task_words(c, dcap);
       const size_t qneed = QUEUE_HDR + (size_t)QUEUE_CAP * 4 + (size_t)QUEUE_CAP * words * 8;
@@ -1506,6 +1570,14 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     if (share_q && (r = queue_launch_init(a.q, s, &launches))) return r;
     return bk_launch(c, wbits, a, grid, block, smem, s, &launches);
   };
+  // a full device: the rows go, and what the call's searches have outgrown
+  auto drop = [&]() -> bool {
+    const bool any = drop_rows(g, s) || !retired.empty();
+    if (cudaStreamSynchronize(s) != cudaSuccess) return false;
+    for (void *q : retired) cudaFree(q);
+    retired.clear();
+    return any;
+  };
   // a part's search, once its preparation is done
   auto search = [&](int p) -> int {
     MCE_CUDA(cudaEventSynchronize(g->part_done[p]));
@@ -1529,32 +1601,44 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     for (int c = 0; c < NCLS && c < 8; ++c) st.class_roots[c] += sh.cls_cnt[c];
     if ((int32_t)sh.max_dplus > st.max_later_degree) st.max_later_degree = (int32_t)sh.max_dplus;
     if ((int64_t)sh.max_deg > st.max_degree) st.max_degree = sh.max_deg;
-    const int64_t arc0 = P.ao_h[P.g[p]], arc1 = P.ao_h[P.g[p + 1]];
-    const int64_t wf = wide_first(arc0, p);
-    if ((rc = run_enc(g, sh, g->roots + vbeg, g->part_shape + p, 1 + p, g->wide_list + wf,
-                      g->wide_off + wf, arc0, arc1, vbeg, vb[p + 1], s, &launches)))
-      return rc;
-    trace_mark(g, s, "rows", p);
-    if (n32 <= 0) return MCE_OK;
     const int dcap = 32, xcap = 1;
     int rxcap = REG_XCAP;
     while (rxcap < (int)sh.max_dminus_reg && rxcap < REG_XCAP_MAX) rxcap <<= 1;
     int grid = 0, block = 0, smem = 0, pc = 1, dm = 0, da = 0;
     QueueView qv;
-    if ((rc = plan(CLS_R32, n32, dcap, xcap, rxcap, &grid, &block, &smem, &pc, &dm, &da, &qv)))
+    bool lanes = false;
+    auto reserve = [&]() -> int {  // what the part's search cannot do without
+      int r = plan(CLS_R32, n32, dcap, xcap, rxcap, &grid, &block, &smem, &pc, &dm, &da, &qv);
+      lanes = use_lanes(o, sh.cls_cnt[CLS_R32], pc, false);
+      if (!r && lanes && !g->lane_resume)
+        r = dalloc(&g->lane_resume, (size_t)RESUME_CAP * RESUME_WORDS);
+      return r;
+    };
+    // rows: as in count_impl, before the host's planning unless they must grow
+    const bool grow = sh.wide_words > g->wide_cap[1 + p];
+    uint64_t granted = g->wide_cap[1 + p];
+    auto build_rows = [&]() -> int {
+      const int64_t arc0 = P.ao_h[P.g[p]], arc1 = P.ao_h[P.g[p + 1]];
+      const int64_t wf = wide_first(arc0, p);
+      const int r = run_enc(g, sh, g->roots + vbeg, g->part_shape + p, 1 + p, g->wide_list + wf,
+                            g->wide_off + wf, arc0, arc1, vbeg, vb[p + 1], granted, s, &launches);
+      trace_mark(g, s, "rows", p);
+      return r;
+    };
+    if (!grow && (rc = build_rows())) return rc;
+    if (n32 > 0 && (rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
+    if (grow && ((rc = rows_grant(g, 1 + p, sh.wide_words, 0, &granted)) || (rc = build_rows())))
       return rc;
+    if (n32 <= 0) return MCE_OK;
     BKArgs a;
     base_args(a, dcap, xcap, rxcap);
     a.roots = g->roots + vbeg;
     a.shape = g->part_shape + p;
     a.fetch = g->part_fetch + 8 * p;
     trace_mark(g, s, "sb", p);
-    if (use_lanes(o, sh.cls_cnt[CLS_R32], pc, false)) {
-      if (!g->lane_resume && (rc = dalloc(&g->lane_resume, (size_t)RESUME_CAP * RESUME_WORDS)))
-        return rc;
-      if ((rc = run_lanes(g, a, &g->part_shape[p].cls_cnt[CLS_R32], vbeg, 1 + p, s, &launches)))
-        return rc;
-    }
+    if (lanes &&
+        (rc = run_lanes(g, a, &g->part_shape[p].cls_cnt[CLS_R32], vbeg, 1 + p, s, &launches)))
+      return rc;
     if ((rc = run_class(CLS_R32, a, grid, block, smem, pc, dm, da, qv, dcap, xcap, rxcap)))
       return rc;
     trace_mark(g, s, "se", p);
@@ -1622,29 +1706,27 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       int grid[2] = {0}, block[2] = {0}, smem[2] = {0}, pc[2] = {1, 1}, dm[2] = {0}, da[2] = {0};
       QueueView qv[2];
       std::vector<WideLaunch> wl;
-      if (ncls[1] > 0 && (rc = plan_wide(g, o, o.bucket_warps_per_root[CLS_MEM]
-                                                   ? o.bucket_warps_per_root[CLS_MEM]
-                                                   : o.warps_per_root,
-                                         false, dcap, xcap, &wl)))
-        return finish(rc);
-      for (int i = 0; i < 2; ++i)
-        if (ncls[i] > 0 && (rc = plan(cls_of[i], ncls[i], dcap, xcap, rxcap, &grid[i], &block[i],
-                                      &smem[i], &pc[i], &dm[i], &da[i], &qv[i])))
-          return finish(rc);
+      const int wide_parts = o.bucket_warps_per_root[CLS_MEM] ? o.bucket_warps_per_root[CLS_MEM]
+                                                              : o.warps_per_root;
+      auto reserve = [&]() -> int {
+        int r = MCE_OK;
+        wl.clear();
+        if (ncls[1] > 0) r = plan_wide(g, o, wide_parts, false, dcap, xcap, &wl);
+        for (int i = 0; i < 2 && !r; ++i)
+          if (ncls[i] > 0)
+            r = plan(cls_of[i], ncls[i], dcap, xcap, rxcap, &grid[i], &block[i], &smem[i], &pc[i],
+                     &dm[i], &da[i], &qv[i]);
+        for (const WideLaunch &l : wl)
+          if (!r) r = grow_slab((size_t)l.grid * 4 * l.slab_words * 8);
+        return r;
+      };
+      if ((rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return finish(rc);
       BKArgs a;
       base_args(a, dcap, xcap, rxcap);
       a.roots = dlist;
       a.shape = sh_final;
       a.fetch = g->part_fetch + 8 * MAX_PARTS;
       for (const WideLaunch &l : wl) {  // wide, then 64-bit
-        const size_t need = (size_t)l.grid * 4 * l.slab_words * 8;
-        if (need > g->slab_bytes) {  // earlier searches of the call keep the old slab
-          if (g->slab) retired.push_back(g->slab);
-          g->slab = nullptr;
-          g->slab_bytes = 0;
-          if ((rc = dalloc((char **)&g->slab, need))) return finish(rc);
-          g->slab_bytes = need;
-        }
         if (!l.W) {
           a.d_lo = l.d_lo;
           if ((rc = run_class(CLS_MEM, a, l.grid, l.block, 0, pc[1], dm[1], da[1], qv[1], dcap, xcap,
