@@ -524,7 +524,7 @@ def run_mine(args, rank, world, local_rank):
         "gpu_launches": int(sum(s_["kernel_launches"] for s_ in stats)),
         # the search (all engine launches of a step) against HBM by its
         # stage-B algorithmic bytes
-        "roofline": {"bound": "hbm", "kernel": "search (bk_*_kernel launches of one step)",
+        "roofline": {"bound": "hbm", "kernel": "search (row pass and engine launches of one step)",
                      "achieved": ach_b, "peak": hbm, "unit": "GB/s", "frac": ach_b / hbm,
                      "traffic": prof.get("search_dram_bytes"),
                      "traffic_note": prof_note or "ncu, profiles/traffic.json",

@@ -117,8 +117,10 @@ typedef struct mce_opts {
                                logs, listing, L2); 8 = its 64-register variant */
   int32_t wait_limit_ms;    /* 0 = default (30 s): a search warp waiting for
                                subtrees gives up after this long without
-                               progress anywhere and the call returns
-                               MCE_ETIMEOUT (the device stays usable)       */
+                               progress anywhere (one waiting for its place
+                               in the task queue: after this long) and the
+                               call returns MCE_ETIMEOUT (the device stays
+                               usable)                                      */
   int32_t count_ops;        /* 1 = run the counting variants of the engines:
                                mce_stats_t.word_ops gets the algorithmic
                                32-bit word operations of the IP walk (per

@@ -116,8 +116,8 @@ struct mce_graph {
   cudaEvent_t seg_fork[1 + MAX_BATCH_PARTS] = {nullptr};
   cudaEvent_t seg_join[2][1 + MAX_BATCH_PARTS] = {{nullptr}};
   // a batch searched part by part as it arrives (mce_batch_count_host):
-  // per part its roots' summary and its search's (device and pinned host),
-  // root fetch counters and sort scratch; the same for the deferred search
+  // per part its roots' summary (device and pinned host), root fetch counters
+  // and sort scratch; a summary and counters for the deferred search
   ShapeInfo *part_shape = nullptr, *part_shape_h = nullptr;
   uint32_t *part_fetch = nullptr;
   void *part_tmp[MAX_BATCH_PARTS] = {nullptr};
@@ -249,7 +249,6 @@ struct BatchParts {
   const int64_t *vo_h, *ao_h;           // host: the layout
 };
 
-// the most vertices of a graph of part p
 // The per-graph peel's size class of a graph of n vertices: 0 more than
 // PEEL_MID_N, 1 more than PEEL_SMALL_N, 2 the rest.
 inline int peel_class(int64_t n) { return n > PEEL_MID_N ? 0 : n > PEEL_SMALL_N ? 1 : 2; }
@@ -322,6 +321,7 @@ int seg_side(mce_graph *g, int i, PeelSide *ps) {
   return MCE_OK;
 }
 
+// the most vertices of a graph of part p
 inline int64_t part_max_n(const BatchParts &P, int p) {
   int64_t mx = 0;
   for (int64_t g = P.g[p]; g < P.g[p + 1]; ++g) {
@@ -879,10 +879,6 @@ int mce_split_csr(mce_graph_t g, int32_t *split_out, int32_t *col_out) {
 }
 
 }  // extern "C"
-
-namespace {
-
-}  // namespace
 
 struct mce_model {
   int device = 0;

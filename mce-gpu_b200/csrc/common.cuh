@@ -123,31 +123,4 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
   return true;
 }
 
-// Binary search in a sorted int array: index of key in [lo, hi) or -1.
-__device__ __forceinline__ int32_t bsearch_idx(const int32_t *a, int32_t lo, int32_t hi,
-                                               int32_t key) {
-  while (lo < hi) {
-    const int32_t mid = (lo + hi) >> 1;
-    const int32_t v = a[mid];
-    if (v == key) return mid;
-    if (v < key)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return -1;
-}
-
-// Branch-free lower bound over a small sorted array (length n <= 2^k).
-__device__ __forceinline__ int32_t lower_bound_small(const int32_t *a, int32_t n, int32_t key) {
-  int32_t lo = 0, len = n;
-  while (len > 0) {
-    const int32_t half = len >> 1;
-    const bool right = a[lo + half] < key;
-    lo = right ? lo + half + 1 : lo;
-    len = right ? len - half - 1 : half;
-  }
-  return lo;
-}
-
 }  // namespace mce
