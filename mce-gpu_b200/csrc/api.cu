@@ -69,6 +69,7 @@ struct mce_graph {
   unsigned long long *wide[1 + MAX_BATCH_PARTS] = {nullptr};  // the wide roots' rows, indexed as enc_next
   uint64_t wide_cap[1 + MAX_BATCH_PARTS] = {0};               // ... and the words they hold
   bool wide_all = true;  // every wide root of the current call has its rows
+  bool no_rows = false;  // the call runs again on a full device: without them
   ShapeInfo *shape = nullptr;
   void *sort_tmp = nullptr;
   size_t sort_tmp_bytes = 0;
@@ -210,6 +211,7 @@ int alloc_graph_bufs(mce_graph *g, int64_t n, int64_t m) {
   const int rc = ar.alloc(&g->arena);
   if (rc) {
     free_graph_bufs(g);
+    g->n = g->m = 0;  // an empty graph until the next upload
     return rc;
   }
   g->cap_n = n;
@@ -349,10 +351,29 @@ int check_args(const int32_t *row_ptr, const int32_t *col, int64_t n, int64_t m)
   return MCE_OK;
 }
 
+// Runs f, which allocates, for handle g; if the device is full, once more after
+// every region of rows was given back, and without rows.
+template <typename F>
+int without_rows_if_full(mce_graph *g, cudaStream_t s, F f) {
+  g->no_rows = false;
+  return reserve_or_drop(MCE_ENOMEM, f, [&]() {
+    (void)cudaGetLastError();  // the allocation that failed
+    bool any = false;
+    for (int j = 0; j < 1 + MAX_PARTS; ++j) any = any || g->wide[j];
+    if (!any || cudaStreamSynchronize(s) != cudaSuccess) return false;
+    for (int j = 0; j < 1 + MAX_PARTS; ++j) {
+      dfree(g->wide[j]);
+      g->wide_cap[j] = 0;
+    }
+    g->no_rows = true;
+    return true;
+  });
+}
+
 int upload_csr(mce_graph *g, const int32_t *row_ptr, const int32_t *col, int64_t n, int64_t m,
                cudaStream_t s) {
   if (n > g->cap_n || m > g->cap_m) {
-    int rc = alloc_graph_bufs(g, n, m);
+    int rc = without_rows_if_full(g, s, [&]() { return alloc_graph_bufs(g, n, m); });
     if (rc) return rc;
   }
   g->n = n;
@@ -496,8 +517,8 @@ constexpr uint32_t SHARE_MIN_LATER = 16;
 // Words of wide roots' rows that region i may have (scratch.h) for a call that
 // allocates `needed` bytes more.
 int rows_grant(mce_graph *g, int i, uint64_t words, uint64_t needed, uint64_t *granted) {
-  *granted = words;
-  if (8 * words <= WIDE_UNASKED) return MCE_OK;
+  *granted = g->no_rows ? 0 : words;
+  if (8 * *granted <= WIDE_UNASKED) return MCE_OK;
   uint64_t others = 0;
   for (int j = 0; j < 1 + MAX_PARTS; ++j)
     if (j != i) others += 8 * g->wide_cap[j];
@@ -505,21 +526,6 @@ int rows_grant(mce_graph *g, int i, uint64_t words, uint64_t needed, uint64_t *g
   MCE_CUDA(cudaMemGetInfo(&free_now, &all));
   *granted = wide_grant(8 * words, 8 * g->wide_cap[i], others, free_now, needed) / 8;
   return MCE_OK;
-}
-
-// Gives every region of rows back (the search then encodes the wide roots
-// itself); false if there was none.
-bool drop_rows(mce_graph *g, cudaStream_t s) {
-  (void)cudaGetLastError();  // the allocation that failed
-  bool any = false;
-  for (int j = 0; j < 1 + MAX_PARTS; ++j) any = any || g->wide[j];
-  if (!any || cudaStreamSynchronize(s) != cudaSuccess) return false;
-  for (int j = 0; j < 1 + MAX_PARTS; ++j) {
-    dfree(g->wide[j]);
-    g->wide_cap[j] = 0;
-  }
-  g->wide_all = false;
-  return cudaMemsetAsync(g->wptr, 0, sizeof(*g->wptr) * ((size_t)g->n + 1), s) == cudaSuccess;
 }
 
 // The rows of every root of a summary (part i - 1 of a batch, or i = 0: the
@@ -991,9 +997,13 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
   if ((rc = read_shape(g, s))) return rc;
   const ShapeInfo &sh = g->shape_h;
   if (sh.cls_cnt[CLS_BIG]) return MCE_ELIMIT;
-  // A few thousand narrow roots without hubs are encoded by the search's own
-  // warps: building their rows first would only add launches (ER n = 200 254
-  // against 236 us, n = 10,000 461 against 441 us a call).
+  // Few narrow roots without hubs are encoded by the search's own warps:
+  // building their rows first mostly adds launches.  ER graphs of mean degree
+  // 8, 20 and 40, us a call with rows first and without: n = 2,000 253, 278, 387
+  // and 238, 263, 373; n = 10,000 423, 436, 669 and 398, 415, 660; n = 24,000
+  // 422, 499, 665 and 387, 469, 663; n = 100,000 543, 686, 1,022 and 503, 650,
+  // 1,088.  So the sides cross by the length of the lists (about 30 later
+  // neighbours) rather than at this line, which costs short lists 7 %.
   const bool rows = sh.wide_cnt > 0 || sh.cls_cnt[CLS_R32] >= ROWS_MIN_ROOTS ||
                     sh.max_dminus_reg > ROWS_MAX_EARLIER;
   // Rows that fit what the handle holds are built at once, beside the host's
@@ -1093,21 +1103,17 @@ int count_impl(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t *his
     }
     return MCE_OK;
   };
-  auto drop = [&]() {
-    granted = 0;
-    return drop_rows(g, s);
-  };
   if (grow) {  // do all of them fit beside the slab of launches for roots with rows?
     if ((rc = plan())) return rc;
     const uint64_t needed = slab_need > g->slab_bytes ? slab_need - g->slab_bytes : 0;
     if ((rc = rows_grant(g, 0, sh.wide_words, needed, &granted))) return rc;
     g->wide_all = granted >= sh.wide_words;
   }
-  if ((rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
+  if ((rc = reserve())) return rc;
   if (grow) {
     const bool planned = g->wide_all;
     if ((rc = build_rows())) return rc;
-    if (g->wide_all != planned && (rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
+    if (g->wide_all != planned && (rc = reserve())) return rc;
   }
   g->wlog_count = o.warp_log ? wlog_total : 0;
   BKArgs a;
@@ -1497,7 +1503,13 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     if (g->slab) retired.push_back(g->slab);  // earlier searches of the call keep the old one
     g->slab = nullptr;
     g->slab_bytes = 0;
-    MCE_CUDA(cudaMalloc((void **)&g->slab, need));
+    if (cudaMalloc((void **)&g->slab, need) != cudaSuccess) {  // without the outgrown ones, then
+      (void)cudaGetLastError();
+      MCE_CUDA(cudaStreamSynchronize(s));
+      for (void *q : retired) cudaFree(q);
+      retired.clear();
+      MCE_CUDA(cudaMalloc((void **)&g->slab, need));
+    }
     g->slab_bytes = need;
     return MCE_OK;
   };
@@ -1566,14 +1578,6 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     if (share_q && (r = queue_launch_init(a.q, s, &launches))) return r;
     return bk_launch(c, wbits, a, grid, block, smem, s, &launches);
   };
-  // a full device: the rows go, and what the call's searches have outgrown
-  auto drop = [&]() -> bool {
-    const bool any = drop_rows(g, s) || !retired.empty();
-    if (cudaStreamSynchronize(s) != cudaSuccess) return false;
-    for (void *q : retired) cudaFree(q);
-    retired.clear();
-    return any;
-  };
   // a part's search, once its preparation is done
   auto search = [&](int p) -> int {
     MCE_CUDA(cudaEventSynchronize(g->part_done[p]));
@@ -1622,7 +1626,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
       return r;
     };
     if (!grow && (rc = build_rows())) return rc;
-    if (n32 > 0 && (rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return rc;
+    if (n32 > 0 && (rc = reserve())) return rc;
     if (grow && ((rc = rows_grant(g, 1 + p, sh.wide_words, 0, &granted)) || (rc = build_rows())))
       return rc;
     if (n32 <= 0) return MCE_OK;
@@ -1716,7 +1720,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
           if (!r) r = grow_slab((size_t)l.grid * 4 * l.slab_words * 8);
         return r;
       };
-      if ((rc = reserve_or_drop(MCE_ENOMEM, reserve, drop))) return finish(rc);
+      if ((rc = reserve())) return finish(rc);
       BKArgs a;
       base_args(a, dcap, xcap, rxcap);
       a.roots = dlist;
@@ -1802,7 +1806,9 @@ int mce_count(mce_graph_t g, const mce_opts_t *opts, uint64_t *total, uint64_t *
     o = *opts;
   else
     mce_opts_default(&o);
-  return count_impl(g, o, total, hist, stats, nullptr);
+  return without_rows_if_full(g, pick_stream(g, o.stream), [&]() {
+    return count_impl(g, o, total, hist, stats, nullptr);
+  });
 }
 
 int mce_list(mce_graph_t g, const mce_opts_t *opts, int32_t *ids_out, int64_t ids_cap,
@@ -1819,10 +1825,13 @@ int mce_list(mce_graph_t g, const mce_opts_t *opts, int32_t *ids_out, int64_t id
   // the records hold a size word per clique beside the ids
   const unsigned long long cap = (unsigned long long)ids_cap + (unsigned long long)cliques_cap;
   ListCtx lc{nullptr, nullptr, cap};
-  int rc = dalloc(&lc.buf, (size_t)(cap > 0 ? cap : 1));
-  if (!rc) rc = dalloc(&lc.words, 1);
   uint64_t total = 0;
-  if (!rc) rc = count_impl(g, o, &total, nullptr, nullptr, nullptr, &lc);
+  int rc = without_rows_if_full(g, pick_stream(g, o.stream), [&]() {
+    int r = MCE_OK;
+    if (!lc.buf) r = dalloc(&lc.buf, (size_t)(cap > 0 ? cap : 1));
+    if (!r && !lc.words) r = dalloc(&lc.words, 1);
+    return r ? r : count_impl(g, o, &total, nullptr, nullptr, nullptr, &lc);
+  });
   unsigned long long words = 0;
   if (!rc && cudaMemcpy(&words, lc.words, sizeof(words), cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = MCE_ECUDA;
@@ -1951,6 +1960,8 @@ void batch_free_bufs(mce_batch *b) {
 int batch_alloc(mce_batch *b, int32_t G, int64_t n, int64_t m) {
   mce_graph *g = b->g;
   int rc;
+  b->G = 0;  // an empty batch, should an allocation fail
+  g->n = g->m = 0;
   if (n > g->cap_n || m > g->cap_m) {
     if ((rc = alloc_graph_bufs(g, n, m))) return rc;
   }
@@ -1979,7 +1990,7 @@ int batch_alloc(mce_batch *b, int32_t G, int64_t n, int64_t m) {
 int batch_load(mce_batch *b, const int32_t *row_ptr, const int32_t *col, const int64_t *vo,
                const int64_t *ao, int32_t G, int64_t n, int64_t m, cudaStream_t s) {
   mce_graph *g = b->g;
-  int rc = batch_alloc(b, G, n, m);
+  int rc = without_rows_if_full(g, s, [&]() { return batch_alloc(b, G, n, m); });
   if (rc) return rc;
   const int64_t rows = n + G;
   MCE_CUDA(cudaMemcpyAsync(b->rp_local, row_ptr, sizeof(int32_t) * (size_t)rows,
@@ -2071,7 +2082,9 @@ int mce_batch_count(mce_batch_t b, const mce_opts_t *opts, uint64_t *per_graph_t
   bc.max_n = b->max_n;
   bc.g_big = b->g_big;
   bc.g_mid = b->g_mid;
-  return count_impl(b->g, o, total, hist, stats, &bc);
+  return without_rows_if_full(b->g, pick_stream(b->g, o.stream), [&]() {
+    return count_impl(b->g, o, total, hist, stats, &bc);
+  });
 }
 
 int mce_batch_count_host(mce_batch_t b, const int32_t *row_ptr, const int32_t *col,
@@ -2098,7 +2111,9 @@ int mce_batch_count_host(mce_batch_t b, const int32_t *row_ptr, const int32_t *c
   // latency (its orientation and sort wait for the search before it) whatever
   // its size: 12.5 to 12.9 ms for 1,024 graphs of 65 M arcs against 15.1 with
   // six parts, 13.4 to 14.0 with four and 12.8 to 13.0 with two (10 and 54).
-  // Otherwise they are six equal ones.
+  // Smaller batches pay that latency without gaining: ms in one part, three
+  // and six for 1.4 M arcs 2.0, 2.5 and 3.7, 5.2 M 3.3, 4.0 and 5.4, 16 M 4.3,
+  // 4.5 and 5.9.  Otherwise they are six equal ones.
   const bool pipelined = !o.log_roots && !o.warp_log && !o.count_ops &&
                          (o.sched == MCE_SCHED_PLAIN || o.sched == MCE_SCHED_DEGREE);
   static const int64_t kGeo[] = {6, 22, 64};  // cumulative 64ths
@@ -2119,7 +2134,7 @@ int mce_batch_count_host(mce_batch_t b, const int32_t *row_ptr, const int32_t *c
            : mce_batch_count(b, &o, per_graph_total, total, hist, stats);
   MCE_CUDA(cudaSetDevice(b->g->device));
   cudaStream_t s = pick_stream(b->g, o.stream);
-  if ((rc = batch_alloc(b, G, n, m))) return rc;
+  if ((rc = without_rows_if_full(b->g, s, [&]() { return batch_alloc(b, G, n, m); }))) return rc;
   if (!b->copy) MCE_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
   if (!b->start) MCE_CUDA(cudaEventCreateWithFlags(&b->start, cudaEventDisableTiming));
   for (int p = 0; p < MAX_PARTS; ++p)
@@ -2168,8 +2183,10 @@ int mce_batch_count_host(mce_batch_t b, const int32_t *row_ptr, const int32_t *c
   bc.max_n = b->max_n;
   bc.g_big = b->g_big;
   bc.g_mid = b->g_mid;
-  rc = pipelined ? count_pipelined(b->g, o, total, hist, stats, &bc)
-                 : count_impl(b->g, o, total, hist, stats, &bc);
+  rc = without_rows_if_full(b->g, s, [&]() {
+    return pipelined ? count_pipelined(b->g, o, total, hist, stats, &bc)
+                     : count_impl(b->g, o, total, hist, stats, &bc);
+  });
   trace_dump(b->g);
   if (rc) cudaStreamSynchronize(b->copy);  // no copy outlives a failed call
   return rc;

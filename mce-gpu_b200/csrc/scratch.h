@@ -30,9 +30,9 @@ inline uint64_t wide_grant(uint64_t want, uint64_t held, uint64_t others, uint64
   return std::max(held, std::min(want, std::min(bound, room)));
 }
 
-// Runs reserve(), which allocates what a call needs and may be run again; if
-// the device is full (code `full`), once more after drop() has given the rows
-// back (false: there were none).
+// Runs reserve(), which allocates and may be run again; if the device is full
+// (code `full`), once more after drop() has given the rows back (false: there
+// were none).
 template <typename Reserve, typename Drop>
 int reserve_or_drop(int full, Reserve reserve, Drop drop) {
   const int rc = reserve();
