@@ -628,10 +628,18 @@ int read_shape(mce_graph *g, cudaStream_t s) {
   return MCE_OK;
 }
 
-// Queue of class c laid out in one buffer: header | seq[cap] | payload.
+// Queue of class c laid out in one buffer: header | seq[cap] | payload.  The
+// wide class's tasks are bk_mem_kernel's or, shorter or (with no root of more
+// than 64 later neighbours) longer, the wide engines'.
+inline uint32_t queue_slot(int c, uint32_t words) {
+  return c == CLS_MEM ? std::max(words, WIDE_TASK_WORDS) : words;
+}
+inline size_t queue_bytes(int c, uint32_t words) {
+  return QUEUE_HDR + (size_t)QUEUE_CAP * (4 + 8 * (size_t)queue_slot(c, words));
+}
 int ensure_queue(mce_graph *g, int c, uint32_t words, QueueView *out) {
   const size_t hdr = QUEUE_HDR, seq = (size_t)QUEUE_CAP * 4;
-  const size_t need = hdr + seq + (size_t)QUEUE_CAP * words * 8;
+  const size_t need = queue_bytes(c, words);
   if (need > g->qbytes[c]) {
     dfree(g->qbuf[c]);
     g->qbytes[c] = 0;
@@ -644,6 +652,7 @@ int ensure_queue(mce_graph *g, int c, uint32_t words, QueueView *out) {
   out->pay = (unsigned long long *)(b + hdr + seq);
   out->cap = QUEUE_CAP;
   out->words = words;
+  out->slot = queue_slot(c, words);
   return MCE_OK;
 }
 
@@ -1533,8 +1542,7 @@ int count_pipelined(mce_graph *g, const mce_opts_t &o, uint64_t *total, uint64_t
     if ((r = grow_slab((size_t)warps * bk_slab_words(c, dcap, xcap, rxcap) * 8))) return r;
     if (share_q) {
       const uint32_t words = bk_task_words(c, dcap);
-      const size_t qneed = QUEUE_HDR + (size_t)QUEUE_CAP * 4 + (size_t)QUEUE_CAP * words * 8;
-      if (qneed > g->qbytes[c] && g->qbuf[c]) {  // ensure_queue would free it in use
+      if (queue_bytes(c, words) > g->qbytes[c] && g->qbuf[c]) {  // ensure_queue would free it in use
         retired.push_back(g->qbuf[c]);
         g->qbuf[c] = nullptr;
         g->qbytes[c] = 0;

@@ -24,9 +24,9 @@
 //
 // What bounds it: instruction issue (77 % of the slots, L1 65 % busy on 512
 // Chung-Lu graphs of 28 M arcs; on 1,024 graphs of 65 M arcs 2.1 ms for the
-// narrow roots, 0.46 ms for the wide ones), most of it the lookups of list elements that are not in the
-// hash - hence the bitmap before it (2.43 -> 2.08 ms) and two windows per
-// step.  It took the place of the search's own encode and the hub rows: the
+// narrow roots, 0.46 ms for the wide ones), most of it the lookups of list
+// elements that are not in the hash - hence the bitmap before it (2.43 -> 2.08
+// ms) and two windows per step.  It took the place of the search's own encode and the hub rows: the
 // search of those graphs' 32-bit class 6.4 -> 4.0 ms, BA n = 1e6 5.3 -> 3.8
 // ms a call, R-MAT 13 59.7 -> 29.1 ms (a taken subtree reads its rows).
 #include <algorithm>

@@ -210,8 +210,9 @@ int lane_launch(const BKArgs &b, const uint32_t *count, int32_t *mid, int32_t *r
 // ---- wide engine of up to 64 W later neighbours, W = 2 or 4 (wide.cu) ------------
 int wide_plan(int W, bool xp, int sms, int xcap, int *grid, size_t *slab_words);
 // The roots of CLS_MEM with d+ in (d_lo, 64 W]; fetch: the launch's root
-// counter.  a.q: a ring for tasks of the class (bk_task_words), used with this
-// engine's own, shorter ones.
+// counter.  a.q: a ring with room for WIDE_TASK_WORDS a task, used with this
+// engine's own tasks (bk_mem_kernel's are bk_task_words long).
+constexpr uint32_t WIDE_TASK_WORDS = 1 + 3 * 4;
 int wide_launch(int W, bool xp, const BKArgs &a, int d_lo, int fetch, int grid, cudaStream_t s,
                 int *launches);
 

@@ -41,6 +41,7 @@ struct QueueView {
   unsigned long long *pay = nullptr; // cap x words
   uint32_t cap = 0;                  // power of two
   uint32_t words = 0;                // u64 words per task
+  uint32_t slot = 0;                 // ... and the most that `pay` has room for
 };
 
 __global__ void queue_init_kernel(QueueView q);

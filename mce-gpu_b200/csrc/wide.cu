@@ -87,7 +87,7 @@ struct WSmem {
 // so that a lane of the taker holds one word.
 template <int W>
 constexpr uint32_t wide_task_words() {
-  static_assert(1 + 3 * W <= 32, "one word per lane");
+  static_assert(1 + 3 * W <= WIDE_TASK_WORDS && WIDE_TASK_WORDS <= 32, "one word per lane");
   return 1 + 3 * W;
 }
 
@@ -538,10 +538,9 @@ int wide_plan(int W, bool xp, int sms, int xcap, int *grid, size_t *slab_words) 
 int wide_launch(int W, bool xp, const BKArgs &args, int d_lo, int fetch, int grid, cudaStream_t s,
                 int *launches) {
   BKArgs a = args;
-  if (a.q.hdr) {  // the ring's slots are sized for the graph's widest root: at least as long
-    const uint32_t words = W == 2 ? wide_task_words<2>() : wide_task_words<4>();
-    if (a.q.words < words) return MCE_EINVAL;
-    a.q.words = words;
+  if (a.q.hdr) {
+    a.q.words = W == 2 ? wide_task_words<2>() : wide_task_words<4>();
+    if (a.q.slot < a.q.words) return MCE_EINVAL;
   }
   const size_t smem = (W == 2 ? sizeof(WSmem<2>) : sizeof(WSmem<4>)) * (W_BLOCK / 32);
   if (W == 2 && xp)

@@ -32,6 +32,7 @@ int main(int argc, char **argv) {
   a.q.pay = pay.data();
   a.q.cap = cap;
   a.q.words = words;
+  a.q.slot = words;
   auto push = [&](unsigned long long x) { return q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k) { return x + k; }); };
   unsigned long long accepted = 0, taken = 0;
   if (mode == "full") {

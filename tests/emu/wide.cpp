@@ -55,9 +55,9 @@ int main(int argc, char **argv) {
   ull all_nodes[4] = {0};
   uint32_t err[4] = {0}, fetch[8] = {0};
   QueueHdr qh;
-  const uint32_t cap = 1024, task = 1 + 4 * ((dcap + 63) / 64);
+  const uint32_t cap = 1024, task = 1 + 4 * ((dcap + 63) / 64), slot = max(task, WIDE_TASK_WORDS);
   std::vector<uint32_t> seq(cap);
-  std::vector<ull> pay((size_t)cap * task);
+  std::vector<ull> pay((size_t)cap * slot + 1, 0xA5);
   BKArgs a;
   memset(&a, 0, sizeof a);
   a.rp = rp.data();
@@ -85,6 +85,7 @@ int main(int argc, char **argv) {
   a.q.pay = pay.data();
   a.q.cap = cap;
   a.q.words = task;
+  a.q.slot = slot;
   int grid = 0;
   if (wide_plan(W, xp, 1, xcap, &grid, &a.slab_words)) return 1;
   slab.resize((size_t)grid * 4 * a.slab_words);
@@ -92,6 +93,7 @@ int main(int argc, char **argv) {
   memset(&qh, 0, sizeof qh);
   emu::launch(emu::Config(1, 256), [&] { queue_init_kernel(a.q); });
   if (wide_launch(W, xp, a, W == 4 ? 128 : 64, 5, grid, nullptr, nullptr)) return 1;
+  if (pay.back() != 0xA5) return 1;
   const ull tail[2] = {err[0], qh.pushed};
   fwrite(count.data(), 8, n, stdout);
   fwrite(nodes.data(), 8, n, stdout);

@@ -8,6 +8,7 @@ import mce_b200 as mce
 import oracle
 from graphs import complete, core
 from test_gpu_lanes import together
+from test_gpu_rows import hub
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +37,22 @@ def test_roots_match_oracle(name, kw):
         r = dg.count(x_pivot=1, log_roots=True, **kw)
         assert r.total == tot and np.array_equal(dg.root_counts(), rc_o)
         assert dg.count(level=mce.LEVEL_L2, **kw).total == tot
+
+
+@pytest.mark.parametrize("kw", [{}, SHARED, {"worker_list": mce.WL_OFF}], ids=str)
+def test_wide_class_of_narrow_roots_only(kw):
+    """Hubs with more than 16,384 earlier and few later neighbours: the wide
+    class, in a graph without a root of more than 64 later neighbours."""
+    g = hub(17500, 20, 3)
+    tot, hist, rc_o, rn_o = oracle.roots(g)
+    with mce.Graph.from_host(g) as dg:
+        for graph in (0, 1):
+            r = dg.count(log_roots=True, cuda_graph=graph, **kw)
+            assert r.stats["class_roots"][2] > 0 and 16 < r.stats["max_later_degree"] <= 64
+            assert r.total == tot and np.array_equal(r.hist, hist)
+            assert np.array_equal(dg.root_counts(), rc_o)
+            assert np.array_equal(dg.root_log(), rn_o)
+        assert dg.count(x_pivot=1, **kw).total == tot
 
 
 @pytest.mark.parametrize("name,threshold", [("cores up to 240", 129), ("a core of 680", 257)])

@@ -30,7 +30,7 @@ def search(W, dcap, xp, donate_after=1):
 
 
 @pytest.mark.parametrize("W", [2, 4])
-@pytest.mark.parametrize("dcap", [256, 448, 449, 640, 2048])
+@pytest.mark.parametrize("dcap", [40, 256, 448, 449, 640, 2048])
 def test_shared_subtrees_whatever_the_widest_root(W, dcap):
     count, count_o, nodes, nodes_o, err, pushed = search(W, dcap, False)
     assert err == 0 and pushed > 20
