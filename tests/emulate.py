@@ -11,6 +11,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "mce-gpu_b200", "csrc")
+_DIR = tempfile.TemporaryDirectory(prefix="mce_emu_")
 _LAUNCH = re.compile(r"([A-Za-z_]\w*(?:<[^<>;]*>)?)<<<(.*?)>>>\(([^;]*)\);", re.S)
 _DYNAMIC = re.compile(r"extern __shared__ (?:__align__\(\d+\) )?([\w ]+?) (\w+)\[\];")
 
@@ -52,11 +53,12 @@ def _translate(name, text):
 @functools.lru_cache(maxsize=None)
 def build(harness):
     """The program of emu/<harness>.cpp with the sources it includes."""
-    tmp = tempfile.mkdtemp(prefix="mce_emu_")
+    tmp = os.path.join(_DIR.name, harness + ".src")
+    os.mkdir(tmp)
     for f in os.listdir(CSRC):
         with open(os.path.join(CSRC, f)) as src, open(os.path.join(tmp, f), "w") as dst:
             dst.write(_translate(f, src.read()))
-    exe = os.path.join(tmp, harness)
+    exe = os.path.join(_DIR.name, harness)
     subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-I", tmp, "-I", os.path.join(HERE, "emu"),
                     os.path.join(HERE, "emu", harness + ".cpp"), "-o", exe], check=True)
     return exe
