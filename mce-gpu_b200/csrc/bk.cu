@@ -88,11 +88,11 @@ __global__ void __launch_bounds__(REG_BLOCK, (NR == 1 && sizeof(Word) == 4) ? 6 
       u64 nd = 0, cnt = 0, op = 0;
       if constexpr (L2) {  // -p l2: the root's edges are the units
         reg_l2_units<Word, NR, LIST>(a, sm, sl, rt, h0, cnt, [&](Word Pv, Word Sv, Word XOv) {
-          if (share && q_wants(a.q)) {  // offered to idle warps at once
+          if (share && wants_task(a.q)) {  // offered to idle warps at once
             const u64 w0 = (u64)(uint32_t)rt.r, w1 = (u64)Pv, w3 = (u64)Sv, w4 = (u64)XOv;
             if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) {
                   return k2 == 0 ? w0 : k2 == 1 ? w1 : k2 == 2 ? 0ull : k2 == 3 ? w3 : w4;
-                })) {
+                }) != Q_KEPT) {
               if (EV && lane == 0) warp_record(a)[2] += 1;
               return;
             }
@@ -221,14 +221,14 @@ __global__ void __launch_bounds__(MEM_BLOCK, MINB) bk_mem_kernel(BKArgs a, int c
     if constexpr (L2) {  // -p l2: the root's edges are the units
       const int WM = (a.dcap + 63) >> 6;
       mem_l2_units<LIST>(a, sl, rt, h0, h1, cnt, [&](bool xo_any) {
-        if (share && q_wants(a.q)) {  // offered to idle warps at once
+        if (share && wants_task(a.q)) {  // offered to idle warps at once
           const u64 *F0 = sl.stk;
           if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
                 if (k2 == 0) return (u64)(uint32_t)r;
                 const uint32_t part = (k2 - 1) / WM, w = (k2 - 1) % WM;
                 if ((int)w >= Wr) return 0ull;
                 return part == 0 ? F0[w] : part == 1 ? 0ull : part == 2 ? F0[3 * Wr + w] : sl.xo[w];
-              })) {
+              }) != Q_KEPT) {
             if (EV && lane == 0) warp_record(a)[2] += 1;
             return;
           }

@@ -1140,13 +1140,14 @@ __device__ void reg_tree(const BKArgs &a, RegSmem<Word, NR> &sm, const RegSlab<W
       if (want) {
         const u64 w0 = (u64)(uint32_t)rt.r, w1 = (u64)Pc, w2 = (u64)Xc, w3 = (u64)Sc,
                   w4 = L2 ? (u64)XO : 0ull;
-        if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) {
-              return k2 == 0 ? w0 : k2 == 1 ? w1 : k2 == 2 ? w2 : k2 == 3 ? w3 : w4;
-            })) {
+        const int pushed = q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) {
+          return k2 == 0 ? w0 : k2 == 1 ? w1 : k2 == 2 ? w2 : k2 == 3 ? w3 : w4;
+        });
+        want = pushed == Q_PUSHED;
+        if (pushed != Q_KEPT) {
           if (EV && lane == 0) warp_record(a)[2] += 1;  // opts.warp_log
           continue;
         }
-        want = false;
       }
     }
     MCE_BD(BD_PIVOT);
@@ -1768,16 +1769,17 @@ __device__ void mem_tree(const BKArgs &a, const Slab &sl, const MemRoot &rt, u64
       MCE_BD(BD_QUEUE);
       const int WM = (a.dcap + 63) >> 6;
       const u64 *Cp = C, *Cx = C + Wr, *Cs = C + 3 * Wr;
-      if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
-            if (k2 == 0) return (u64)(uint32_t)rt.r;
-            const uint32_t part = (k2 - 1) / WM, w = (k2 - 1) % WM;
-            if ((int)w >= Wr) return 0ull;
-            return part == 0 ? Cp[w] : part == 1 ? Cx[w] : part == 2 ? Cs[w] : (L2 && XO ? sl.xo[w] : 0ull);
-          })) {
+      const int pushed = q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
+        if (k2 == 0) return (u64)(uint32_t)rt.r;
+        const uint32_t part = (k2 - 1) / WM, w = (k2 - 1) % WM;
+        if ((int)w >= Wr) return 0ull;
+        return part == 0 ? Cp[w] : part == 1 ? Cx[w] : part == 2 ? Cs[w] : (L2 && XO ? sl.xo[w] : 0ull);
+      });
+      want = pushed == Q_PUSHED;
+      if (pushed != Q_KEPT) {
         if (EV && lane == 0) warp_record(a)[2] += 1;  // opts.warp_log
         continue;
       }
-      want = false;
     }
     MCE_BD(BD_PIVOT);
     k = (int)__reduce_max_sync(MCE_FULL, (unsigned)k);

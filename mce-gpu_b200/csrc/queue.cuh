@@ -50,45 +50,53 @@ __global__ void queue_init_kernel(QueueView q);
 // the task there, pos + cap once the task was taken.
 //
 // Claim a position and publish `words` task words held by the warp (lane k
-// holds words k, k+32, ...; supplied by `get(k)`).  Returns false if the ring
-// is full: a position is only claimed while positions run less than a lap,
-// minus one per warp of the launch, ahead of tickets.  Even with every warp
-// past that test at once the position stays less than a lap ahead, so the
-// ticket of its slot's last task is drawn and the wait for the slot is one for
-// a running warp to copy a task out.  That wait is bounded by limit_ns: when it
-// runs out the search ends with MCE_ERR_WAIT_TIMEOUT.  The slot's word is read
-// without acquire (an acquire empties the SM's L1: 1,024 Chung-Lu graphs 9.64
-// ms a count, 9.62 without): nothing is read after it, and the task is written
-// only where it has the awaited value, which its last reader released.
+// holds words k, k+32, ...; supplied by `get(k)`).
+//
+// Positions stay less than a lap ahead of tickets, so that the ticket of a
+// slot's last task is drawn and the wait for the slot is one for a running warp
+// to copy a task out: each claim follows a look at both counters that found
+// positions less than a lap, minus one per warp of the launch, ahead, and each
+// look is good for one claim, so at most every warp claims after the last one.
+// The look is q_wants' or that of the warp's last push, which has it in flight
+// beside the slot's word (with a look of its own before each claim a count of
+// BA n = 1,155 took 1,040 us, with this one 1,023).
+//
+// The wait is bounded by limit_ns: when it runs out the search ends with
+// MCE_ERR_WAIT_TIMEOUT.  The slot's word is read without acquire (an acquire
+// empties the SM's L1: those graphs 9.64 ms a count, 9.62 without): nothing is
+// read after it, and the task is written only where it has the awaited value,
+// which its last reader released.
+enum QPush : int { Q_KEPT = 0, Q_PUSHED = 1, Q_PUSHED_LAST = 2 };  // ... and no room for the next
+
 template <typename Get>
-__device__ __forceinline__ bool q_push(const QueueView &q, uint32_t *err, uint64_t limit_ns,
-                                       Get get) {
+__device__ __forceinline__ int q_push(const QueueView &q, uint32_t *err, uint64_t limit_ns,
+                                      Get get) {
   const uint32_t lane = lane_id();
   uint32_t pos = 0;
-  int ok = 0;
+  int ok = Q_KEPT;
   if (lane == 0) {
-    const int32_t room = (int32_t)q.cap - (int32_t)(gridDim.x * (blockDim.x >> 5));
-    if ((int32_t)(ld_volatile(&q.hdr->tail) - ld_volatile(&q.hdr->head)) < room) {
-      pos = atomicAdd(&q.hdr->tail, 1u);
-      const uint32_t *s = &q.seq[pos & (q.cap - 1)];
-      ok = ld_volatile(s) == pos;
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();
-        do {
-          __nanosleep(64);
-          ok = ld_volatile(s) == pos;
-        } while (!ok && globaltimer_ns() - t0 <= limit_ns);
-      }
-      if (ok) {
-        atomicAdd(&q.hdr->work, 1u);  // counted before anyone can take it
-        atomicAdd(&q.hdr->pushed, 1u);
-      } else {
-        atomicOr(err, MCE_ERR_WAIT_TIMEOUT);
-      }
+    pos = atomicAdd(&q.hdr->tail, 1u);
+    const uint32_t head = ld_volatile(&q.hdr->head);
+    const uint32_t *s = &q.seq[pos & (q.cap - 1)];
+    bool free = ld_volatile(s) == pos;
+    if (!free) {
+      const uint64_t t0 = globaltimer_ns();
+      do {
+        __nanosleep(64);
+        free = ld_volatile(s) == pos;
+      } while (!free && globaltimer_ns() - t0 <= limit_ns);
+    }
+    if (free) {
+      atomicAdd(&q.hdr->work, 1u);  // counted before anyone can take it
+      atomicAdd(&q.hdr->pushed, 1u);
+      const int32_t room = (int32_t)q.cap - (int32_t)(gridDim.x * (blockDim.x >> 5));
+      ok = (int32_t)(pos + 1 - head) < room ? Q_PUSHED : Q_PUSHED_LAST;
+    } else {
+      atomicOr(err, MCE_ERR_WAIT_TIMEOUT);
     }
   }
   ok = __shfl_sync(MCE_FULL, ok, 0);
-  if (!ok) return false;
+  if (ok == Q_KEPT) return ok;
   pos = __shfl_sync(MCE_FULL, pos, 0);
   unsigned long long *dst = q.pay + (size_t)(pos & (q.cap - 1)) * q.words;
   for (uint32_t k = lane; k < q.words; k += 32) dst[k] = get(k);
@@ -98,7 +106,7 @@ __device__ __forceinline__ bool q_push(const QueueView &q, uint32_t *err, uint64
     st_release(&q.seq[pos & (q.cap - 1)], pos + 1);
   }
   __syncwarp();
-  return true;
+  return ok;
 }
 
 // Whether the task of ticket `pos` is there (lane 0's answer).
@@ -119,7 +127,8 @@ __device__ __forceinline__ void q_take(const QueueView &q, uint32_t pos, Put put
   __syncwarp();
 }
 
-// Donate a child only while more warps are waiting than tasks are queued.
+// Donate a child only while more warps are waiting than tasks are queued.  (A
+// look that allows one claim: a ring has more slots than the device warps.)
 __device__ __forceinline__ bool q_wants(const QueueView &q) {
   if (!q.hdr) return false;
   return (int32_t)(ld_volatile(&q.hdr->head) - ld_volatile(&q.hdr->tail)) > 0;

@@ -310,18 +310,18 @@ __device__ void w_tree(const BKArgs &a, WSmem<W> &sm, u64 *slab, const WRoot &rt
         recheck = 32;
       }
       if (want) {
-        if (q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
-              u64 x = (u64)(uint32_t)rt.r;
+        const int pushed = q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k2) -> u64 {
+          u64 x = (u64)(uint32_t)rt.r;
 #pragma unroll
-              for (int j = 0; j < W; ++j) {
-                if ((int)k2 == 1 + j) x = Pc.w[j];
-                if ((int)k2 == 1 + W + j) x = Xc.w[j];
-                if ((int)k2 == 1 + 2 * W + j) x = Sc.w[j];
-              }
-              return x;
-            }))
-          continue;
-        want = false;
+          for (int j = 0; j < W; ++j) {
+            if ((int)k2 == 1 + j) x = Pc.w[j];
+            if ((int)k2 == 1 + W + j) x = Xc.w[j];
+            if ((int)k2 == 1 + 2 * W + j) x = Sc.w[j];
+          }
+          return x;
+        });
+        want = pushed == Q_PUSHED;
+        if (pushed != Q_KEPT) continue;
       }
     }
     if (B.any()) {  // come back to the frame's other branches

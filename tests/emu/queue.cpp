@@ -1,5 +1,6 @@
 // queue MODE: the task ring on the CPU.  Prints what the mode says.
-//   full   a donor that nobody takes from: {accepted, positions handed out}
+//   full   a donor that nobody takes from, a ticket drawn: {accepted, positions
+//          handed out}
 //   laps   two donors and two takers over many laps: {tasks pushed, sum of the
 //          tasks taken}
 //   stale  a taker without work whose slot is still an earlier lap's: {status}
@@ -33,14 +34,19 @@ int main(int argc, char **argv) {
   a.q.cap = cap;
   a.q.words = words;
   a.q.slot = words;
-  auto push = [&](unsigned long long x) { return q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k) { return x + k; }); };
+  auto push = [&](unsigned long long x) {
+    return q_push(a.q, a.err, a.wait_limit_ns, [&](uint32_t k) { return x + k; });
+  };
   unsigned long long accepted = 0, taken = 0;
   if (mode == "full") {
+    hdr.head = 1;
     emu::launch(emu::Config(1, 64), [&] {
       if (threadIdx.x >= 32) return;
-      for (int i = 0; i < 200; ++i) {
-        const bool ok = push(i);
-        if (lane_id() == 0) accepted += ok;
+      bool want = wants_task(a.q);
+      for (int i = 0; i < 200 && want; ++i) {
+        const int pushed = push(i);
+        if (lane_id() == 0) accepted += pushed != Q_KEPT;
+        want = pushed == Q_PUSHED || wants_task(a.q);
       }
     });
     printf("%llu %u\n", accepted, hdr.tail);
@@ -48,8 +54,15 @@ int main(int argc, char **argv) {
     emu::launch(emu::Config(1, 128), [&] {
       if (lane_id() == 0) atomicAdd(&hdr.work, 1u);
       if (threadIdx.x < 64)
-        for (unsigned long long i = 0; i < 1000; ++i) {
-          while (!push(3 * (1000 * (threadIdx.x >> 5) + i))) __nanosleep(1);
+        for (unsigned long long i = 0, want = 0; i < 1000;) {
+          if (!want && !wants_task(a.q)) {
+            __nanosleep(1);
+            continue;
+          }
+          const int pushed = push(3 * (1000 * (threadIdx.x >> 5) + i));
+          if (pushed == Q_KEPT) return;
+          want = pushed == Q_PUSHED;
+          ++i;
           if (lane_id() == 0) ++accepted;
         }
       root_phase_done(a.q);
@@ -70,8 +83,8 @@ int main(int argc, char **argv) {
     seq[0] = 1;
     hdr.head = hdr.tail = cap;
     emu::launch(emu::Config(1, 32), [&] {
-      const bool ok = push(7);
-      if (lane_id() == 0) accepted += ok;
+      const int pushed = push(7);
+      if (lane_id() == 0) accepted += pushed != Q_KEPT;
     });
     printf("%llu %u\n", accepted, err);
   } else {
